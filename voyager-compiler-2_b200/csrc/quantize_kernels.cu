@@ -973,14 +973,17 @@ int vq_dequantize_mx(const void* in, const void* scale, const void* code, int32_
   VQ_REQUIRE(in && out, "vq_dequantize_mx: null argument");
   VQ_REQUIRE(!code || n_code > 0, "vq_dequantize_mx: empty codebook");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (dtype == VQ_BF16 && !code && scale && !global_scale && (n % 8) == 0 && aligned16(in) && aligned16(out)) {
+  // bfloat16 operands of whole vectors with a scale, read directly or through a 16-entry codebook
+  if (dtype == VQ_BF16 && (!code || n_code == 16) && scale && !global_scale && (n % 8) == 0 && aligned16(in) &&
+      aligned16(out)) {
     // dense per-block scales along the last axis: parameter index = flat / block
     int64_t d = 0;
     if (g.ndim == 1 && g.stride[0] == 1) d = g.div[0];
     else if (g.ndim == 2 && g.div[0] == 1 && g.stride[1] == 1 && g.size[1] % g.div[1] == 0 &&
              g.stride[0] == g.size[1] / g.div[1]) d = g.div[1];
     if (d >= 8 && d % 8 == 0 && d < (1ll << 31))
-      return fast_scale_bf16(in, scale, out, n / 8, (uint32_t)(d / 8), st);
+      return code ? fast_decode_scale_bf16(in, code, scale, out, n / 8, (uint32_t)(d / 8), st)
+                  : fast_scale_bf16(in, scale, out, n / 8, (uint32_t)(d / 8), st);
   }
   int grid = grid_for(n, 256, 8);
   VQ_DISPATCH_DTYPE(dtype, (dequantize_mx_kernel<DT><<<grid, 256, 0, st>>>(in, scale, code, n_code, global_scale,

@@ -119,5 +119,7 @@ int fast_quantize_bf16(const void* in, const void* scale, int pdt, void* out, in
                        const Round& r, int fast_mode, cudaStream_t st);
 int fast_scale_bf16(const void* in, const void* scale, void* out, int64_t nvec, uint32_t vecs_per_scale,
                     cudaStream_t st);
+int fast_decode_scale_bf16(const void* in, const void* code, const void* scale, void* out, int64_t nvec,
+                           uint32_t vecs_per_scale, cudaStream_t st);
 
 }  // namespace vq
