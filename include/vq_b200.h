@@ -569,6 +569,13 @@ int vq_gemm_status(int reset);
 int vq_kivi_read_2bit(const void* packed, const void* scale, const void* zero_point, void* out, int64_t outer,
                       int64_t T, int64_t D, int along_channels, int64_t block, void* stream);
 
+/* The KIVI cache write for 2-bit codes, the counterpart of vq_kivi_read_2bit: quantized_ops::quantize_affine(x, uint2
+ * table, axes, block, 0, 3, scale table) (ops/quantized.py:1227-1283) on a bfloat16 [outer, T, D] tensor with the codes
+ * packed as vq_pack_codes packs them, in one pass.  VQ_EUNSUPPORTED unless block is 32, 64 or 128, the groups are
+ * whole and, for groups of positions, D is a multiple of 32 (the caller then runs the two calls). */
+int vq_kivi_write_2bit(const void* in, void* scale, void* zero_point, void* packed, int64_t outer, int64_t T, int64_t D,
+                       int along_channels, int64_t block, const VqRound* scale_round, void* stream);
+
 /* One decode step's attention straight from the packed KIVI cache, for every (sequence, KV head) pair
  * `outer`: the nodes
  *   k = dequantize(k_codes, k_scale, k_zero); v = dequantize(v_codes, v_scale, v_zero)   (as vq_kivi_read_2bit)

@@ -161,3 +161,44 @@ def test_rope_append_equals_the_graph_nodes(per_sequence):
     want_v[:, :, 5].copy_(qkv[:, (hq + hkv) * d:].reshape(B, hkv, d))
     got_q = vb.kivi.rope_append(qkv, cos, sin, hq, k_win, v_win, 5)
     assert torch.equal(got_q, want_q) and torch.equal(k_win, want_k) and torch.equal(v_win, want_v)
+
+
+@pytest.mark.parametrize("shape,axis,block", [((1, 32, 32), -2, 32), ((2, 3, 192, 96), -2, 64), ((1, 256, 128), -2, 128),
+                                              ((128, 160), 0, 64), ((1, 1, 64), -1, 64), ((3, 5, 96), -1, 32),
+                                              ((2, 37, 128), -1, 64), ((2, 9, 384), 2, 128)])
+@pytest.mark.parametrize("special", [False, True])
+@pytest.mark.parametrize("scale_table", [None, "fp8_e4m3"])
+def test_one_pass_write_is_the_two_operators(shape, axis, block, special, scale_table):
+    vb = _vb()
+    g = torch.Generator().manual_seed(sum(shape) + block)
+    x = torch.randn(*shape, generator=g) * torch.exp2(torch.randint(-6, 7, shape[:-1] + (1,), generator=g).float())
+    if special:   # groups of zeros, of one value, of tiny and huge values, with infinities and NaN
+        pick = torch.rand(shape, generator=g)
+        flat = torch.rand(shape[:-1] + (1,), generator=g)
+        x = torch.where(flat < 0.2, torch.zeros(()), x)
+        x = torch.where((flat > 0.2) & (flat < 0.3), torch.full((), -3.75), x)
+        x = torch.where((flat > 0.3) & (flat < 0.4), x * 2.0 ** -128, x)
+        x = torch.where((flat > 0.4) & (flat < 0.5), x * 2.0 ** 118, x)
+        x = torch.where(pick < 2e-3, torch.full((), float("inf")), x)
+        x = torch.where((pick > 2e-3) & (pick < 3e-3), torch.full((), float("-inf")), x)
+        x = torch.where((pick > 3e-3) & (pick < 5e-3), torch.full((), float("nan")), x)
+    x = x.bfloat16().cuda()
+    qmap = vb.get_quantization_map("uint2", "cuda")
+    table = None if scale_table is None else vb.get_quantization_map(scale_table, "cuda")
+    assert vb.kivi._write_2bit(x, qmap, axis, block, table) is not None
+    cache = vb.kivi.quantize_cache(x, qmap, axis, block, 2, table)
+    scale, zero, codes = torch.ops.quantized_ops.quantize_affine(x, qmap, [axis], block, 0.0, 3.0, table)
+    assert torch.equal(cache.scale.view(torch.int16), scale.view(torch.int16))
+    assert torch.equal(cache.zero_point.view(torch.int16), zero.view(torch.int16))
+    assert torch.equal(cache.packed, vb.kivi.pack_codes(codes, 2))
+    want = vb.kivi.unpack_dequantize(cache.packed, 2, shape, scale, zero, block)
+    assert bits_equal(cache.read().cpu(), want.cpu())
+
+
+def test_one_pass_write_leaves_other_layouts_and_grids_alone():
+    vb = _vb()
+    x = torch.randn(2, 100, 64).bfloat16().cuda()
+    uint2, int2 = (vb.get_quantization_map(n, "cuda") for n in ("uint2", "int2"))
+    for args in ((x, uint2, 1, 64), (x, uint2, -2, 50), (x, uint2, 0, 2), (x, int2, -1, 64), (x.float(), uint2, -1, 64),
+                 (x, uint2, 3, 64)):
+        assert vb.kivi._write_2bit(*args, None) is None

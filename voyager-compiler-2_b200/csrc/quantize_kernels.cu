@@ -434,24 +434,6 @@ mx_generic_kernel(const void* __restrict__ in, void* __restrict__ scale_out, voi
 __device__ __forceinline__ float nan_min(float a, float b) { return (a != a || b != b) ? (a + b) : fminf(a, b); }
 __device__ __forceinline__ float nan_max(float a, float b) { return (a != a || b != b) ? (a + b) : fmaxf(a, b); }
 
-template <int DT>
-__device__ __forceinline__ void affine_params(float low, float high, float qmin, float qmax,
-                                              const Round& sr, float* scale, float* zero) {
-  using E = Elem<DT>;
-  float range = E::round(__fsub_rn(high, low));
-  float s = E::round(__fdiv_rn(range, __fsub_rn(qmax, qmin)));
-  s = (s > 0.0f) ? s : 1.0f;
-  if (sr.mode != VQ_ROUND_NONE) {
-    s = E::round(apply_round(sr, s, 0));
-    s = (s > 0.0f) ? s : 1.0f;
-  }
-  float z = E::round(__fdiv_rn(-low, s));
-  z = E::round(__fadd_rn(z, qmin));
-  if (sr.mode != VQ_ROUND_NONE) z = E::round(apply_round(sr, z, 0));
-  *scale = s;
-  *zero = z;
-}
-
 // Blocks of `block` along B in a dense [O, B, I] view; thread per (o, b-block, i).
 template <int DT>
 __global__ void __launch_bounds__(256)

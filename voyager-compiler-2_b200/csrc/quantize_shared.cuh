@@ -89,6 +89,25 @@ __device__ __forceinline__ float block_scale(uint32_t amax_bits, const ScaleRule
   return scale;
 }
 
+// group-wise affine rule: [low, high] -> [qmin, qmax]
+template <int DT>
+__device__ __forceinline__ void affine_params(float low, float high, float qmin, float qmax,
+                                              const Round& sr, float* scale, float* zero) {
+  using E = Elem<DT>;
+  float range = E::round(__fsub_rn(high, low));
+  float s = E::round(__fdiv_rn(range, __fsub_rn(qmax, qmin)));
+  s = (s > 0.0f) ? s : 1.0f;
+  if (sr.mode != VQ_ROUND_NONE) {
+    s = E::round(apply_round(sr, s, 0));
+    s = (s > 0.0f) ? s : 1.0f;
+  }
+  float z = E::round(__fdiv_rn(-low, s));
+  z = E::round(__fadd_rn(z, qmin));
+  if (sr.mode != VQ_ROUND_NONE) z = E::round(apply_round(sr, z, 0));
+  *scale = s;
+  *zero = z;
+}
+
 __device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7FFFFFFFu; }
 
 

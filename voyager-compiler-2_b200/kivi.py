@@ -111,11 +111,43 @@ def _read_2bit(cache: "PackedCache", outer, T, D, along_channels) -> torch.Tenso
     return out
 
 
+@N.device_guarded
+def _write_2bit(x, qmap, axis, block_size, scale_qmap):
+    """The one-pass write, or ``None`` when ``x``'s layout or ``qmap`` (anything but the uint2 grid) is not its."""
+    nd = x.dim()
+    if not x.is_cuda or x.dtype != torch.bfloat16 or nd < 2 or not -nd <= axis < nd or axis % nd < nd - 2 \
+            or x.numel() == 0 or block_size < 1:
+        return None
+    spec = R.table_round(qmap)
+    if spec.mode != N.ROUND_INT or (spec.c.lo, spec.c.hi) != (0.0, 3.0):
+        return None
+    sspec = R.none_round() if scale_qmap is None else R.table_round(scale_qmap)
+    x = x.contiguous()
+    T, D = x.shape[-2:]
+    along_channels = int(axis % nd == nd - 1)
+    if (D if along_channels else T) % block_size:
+        return None
+    shape = list(x.shape)
+    shape[axis] //= block_size
+    scale = torch.empty(shape, dtype=x.dtype, device=x.device)
+    zero_point = torch.empty_like(scale)
+    packed = torch.empty(x.numel() // 4, dtype=torch.uint8, device=x.device)
+    rc = N.lib().vq_kivi_write_2bit(x.data_ptr(), scale.data_ptr(), zero_point.data_ptr(), packed.data_ptr(),
+                                    x.numel() // (T * D), T, D, along_channels, block_size, sspec.ref, _stream())
+    if rc == -3:   # VQ_EUNSUPPORTED
+        return None
+    N.check(rc, "vq_kivi_write_2bit")
+    return PackedCache(packed, scale, zero_point, tuple(x.shape), [axis], block_size, 2)
+
+
 def quantize_cache(x: torch.Tensor, qmap: torch.Tensor, axis: int, block_size: int, bits: int,
                    scale_qmap: Optional[torch.Tensor] = None) -> PackedCache:
     """Quantize ``x`` in groups of ``block_size`` along ``axis`` to unsigned ``bits``-bit codes
     (``quantize_affine``, reference ``ops/quantized.py:1227-1283``) and pack them."""
     axes = [axis]
+    cache = _write_2bit(x, qmap, axis, block_size, scale_qmap) if bits == 2 else None
+    if cache is not None:
+        return cache
     scale, zero_point, codes = Q.quantize_affine(x, qmap, axes, block_size, 0.0, float(2 ** bits - 1), scale_qmap)
     return PackedCache(pack_codes(codes, bits), scale, zero_point, tuple(x.shape), axes, block_size, bits)
 
