@@ -509,12 +509,27 @@ int vq_transpose_quantize_fp8(const void* x, void* out, void* codes, void* amax_
  * vq_quantize_nvfp4 casts bfloat16 [rows, K] with the arithmetic of
  * quantized_ops::quantize_mx (ops/quantized.py:1080-1115) for an e2m1 table,
  * an e4m3 scale table, quant_max 6 and the given global scale (device scalar).
+ * vq_cast_nvfp4 takes the global scale from the tensor itself: amax is one float of device memory, filled by the call
+ * unless amax_given, and t (bfloat16) receives bf16(bf16(amax) / 2688) (calculate_global_scale,
+ * quantization/fake_quantize.py:142-160); a ragged last scale tile is zeroed by the call.
+ * vq_cast_nvfp4_pair casts [M, K] along K and its transpose along M, the transpose's runs of 16 rotated by `matrix`
+ * (16 x 16 float32, or null) and either form stochastically rounded when its seed (device int64) is given
+ * (quantize_nvfp4_pair, backend/gpu/nvfp4.py:953-980); amax: two floats of workspace.
+ * vq_cast_nvfp4_square casts a weight in 16 x 16 blocks, packed both ways (quantize_nvfp4_square, :983-1017); amax: one
+ * float.  Both take extents that are multiples of 64.
  * vq_pack_nvfp4 packs that operator's own outputs (bfloat16-valued codes
  * [rows, K], bfloat16 scales [rows, K/16]) and sets *bad_flag (device int) to 1
  * if a value is not representable (pack_nvfp4, backend/gpu/nvfp4.py:1045-1091). */
 int64_t vq_nvfp4_scale_bytes(int64_t rows, int64_t K);
 int vq_quantize_nvfp4(const void* in, const void* global_scale, int global_scale_dtype, void* codes,
                       void* scales, int64_t rows, int64_t K, void* stream);
+int vq_cast_nvfp4(const void* in, void* amax, int amax_given, void* codes, void* scales, void* t, int64_t rows,
+                  int64_t K, void* stream);
+int vq_cast_nvfp4_pair(const void* in, const float* matrix, const int64_t* seed, const int64_t* seed_t, float* amax,
+                       void* codes, void* scales, void* t, void* codes_t, void* scales_t, void* t_t, int64_t M,
+                       int64_t K, void* stream);
+int vq_cast_nvfp4_square(const void* in, float* amax, void* codes, void* scales, void* codes_t, void* scales_t, void* t,
+                         int64_t N, int64_t K, void* stream);
 int vq_pack_nvfp4(const void* codes_in, const void* scales_in, void* codes, void* scales, int64_t rows,
                   int64_t K, int* bad_flag, void* stream);
 

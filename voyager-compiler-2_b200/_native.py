@@ -131,6 +131,9 @@ SIGNATURES = {
     "vq_pack_lut4": [_P, _P, _I64, _I64, _P, _P],
     "vq_kivi_decode_attention": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I64, _I64, _I64, _F, _P],
     "vq_kivi_write_2bit": [_P, _P, _P, _P, _I64, _I64, _I64, _I, _I64, ctypes.POINTER(VqRound), _P],
+    "vq_cast_nvfp4": [_P, _P, _I, _P, _P, _P, _I64, _I64, _P],
+    "vq_cast_nvfp4_pair": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _P],
+    "vq_cast_nvfp4_square": [_P, _P, _P, _P, _P, _P, _P, _I64, _I64, _P],
     "vq_kivi_read_2bit": [_P, _P, _P, _P, _I64, _I64, _I64, _I, _I64, _P],
     "vq_gptq_block": [_P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I, _F, _F, _I, ctypes.POINTER(VqRound),
                       ctypes.POINTER(VqRound), _P],

@@ -132,6 +132,35 @@ def nvfp4_gemm(a: PackedNVFP4, b: PackedNVFP4, alpha: Optional[torch.Tensor] = N
     return out.reshape(*abatch, m, n)
 
 
+def _matrix_outputs(rows, k, device):
+    """Uninitialised codes, scales and global scale of a matrix's cast (the kernels write every byte)."""
+    return (torch.empty(rows, k // 2, dtype=torch.uint8, device=device),
+            torch.empty(1, int(N.lib().vq_nvfp4_scale_bytes(rows, k)), dtype=torch.uint8, device=device),
+            torch.empty((), dtype=torch.bfloat16, device=device))
+
+
+@N.device_guarded
+def _cast_with_amax(x, amax=None):
+    """``(codes, scales, t)`` of a contiguous bfloat16 matrix: its tensor-wide amax (or the one given, 0-d float32), the
+    global scale and the cast in one call; ``None`` when the kernel does not take ``x``."""
+    if not x.is_cuda or x.dtype != torch.bfloat16 or x.numel() == 0 or x.shape[1] % 64 or x.data_ptr() % 16:
+        return None
+    rows, k = x.shape
+    codes, scales, t = _matrix_outputs(rows, k, x.device)
+    given = amax is not None
+    if not given:
+        amax = torch.empty((), dtype=torch.float32, device=x.device)
+    N.check(N.lib().vq_cast_nvfp4(x.data_ptr(), amax.data_ptr(), int(given), codes.data_ptr(), scales.data_ptr(),
+                                  t.data_ptr(), rows, k, _stream()), "vq_cast_nvfp4")
+    return codes, scales, t
+
+
+def _two_way(x):
+    """Whether the kernels that cast a matrix along both axes take ``x``."""
+    return (x.is_cuda and x.dtype == torch.bfloat16 and x.numel() > 0 and x.shape[0] % 64 == 0 and x.shape[1] % 64 == 0
+            and x.data_ptr() % 16 == 0)
+
+
 @N.device_guarded
 def silu_mul_cast_nvfp4(gate: torch.Tensor, up: torch.Tensor):
     """``quantize_nvfp4(silu(gate) * up)`` with the product and its tensor-wide amax made in one pass:
@@ -142,6 +171,9 @@ def silu_mul_cast_nvfp4(gate: torch.Tensor, up: torch.Tensor):
     if gate.dtype != torch.bfloat16 or up.dtype != torch.bfloat16 or gate.shape != up.shape or gate.dim() != 2:
         raise NotImplementedError("silu_mul_cast_nvfp4 takes two bfloat16 matrices of one shape")
     act, amax = silu_mul_amax(gate, up)
+    fast = _cast_with_amax(act, amax)
+    if fast is not None:
+        return fast
     t = O.global_scale_of_amax(amax, torch.bfloat16, FP4_MAX, E4M3_MAX)
     packed = cast_nvfp4(act, t)
     return packed.codes, packed.scales, t
@@ -192,9 +224,13 @@ def quantize_nvfp4(input: torch.Tensor, axis: int = -1, seed: Optional[torch.Ten
     axis %= input.ndim
     if hadamard is not None:
         input = O.hadamard_rotate(input, axis, hadamard)
-    t = O.calculate_global_scale(input, FP4_MAX, E4M3_MAX)
     moved = input.movedim(axis, -1).contiguous()
     rows = moved.reshape(-1, moved.shape[-1])
+    fast = _cast_with_amax(rows) if seed is None else None
+    if fast is not None:
+        codes, scales, t = fast
+        return codes.view(*moved.shape[:-1], -1), scales, t
+    t = O.calculate_global_scale(input, FP4_MAX, E4M3_MAX)
     if seed is None:
         packed = cast_nvfp4(rows, t)
     else:
@@ -215,10 +251,45 @@ def quantize_nvfp4_pair(input: torch.Tensor, seed: Optional[torch.Tensor] = None
     """``quantize_nvfp4`` of a matrix ``[M, K]`` along its last axis and of its transpose along its last
     axis (with ``hadamard`` and ``transpose_seed``): ``(codes, scales, t, codes_T, scales_T, t_T)``, what
     a training step needs of one operand for its forward and weight-gradient GEMMs
-    (reference ``backend/gpu/nvfp4.py:953-980``).  Two casts here, each reading the matrix once."""
+    (reference ``backend/gpu/nvfp4.py:953-980``): one pass for the two amaxes and one for the two casts where both
+    extents are multiples of 64, two separate casts otherwise."""
     if input.ndim != 2:
         raise ValueError("quantize_nvfp4_pair takes a matrix")
+    if _two_way(input) and (hadamard is None or hadamard.shape == (16, 16)):
+        return _cast_pair(input.contiguous(), seed, transpose_seed, hadamard)
     return (*quantize_nvfp4(input, -1, seed), *quantize_nvfp4(input.mT, -1, transpose_seed, hadamard))
+
+
+@N.device_guarded
+def _cast_pair(x, seed, transpose_seed, hadamard):
+    dev = x.device
+
+    def device_seed(s):
+        return s if s is None or (s.dtype == torch.int64 and s.device == dev) else s.to(device=dev, dtype=torch.int64)
+
+    seed, transpose_seed = device_seed(seed), device_seed(transpose_seed)
+    if hadamard is not None:
+        hadamard = hadamard.to(device=dev, dtype=torch.float32).contiguous()
+    m, k = x.shape
+    codes, scales, t = _matrix_outputs(m, k, dev)
+    codes_t, scales_t, t_t = _matrix_outputs(k, m, dev)
+    amax = torch.empty(2, dtype=torch.float32, device=dev)
+    N.check(N.lib().vq_cast_nvfp4_pair(x.data_ptr(), _ptr(hadamard), _ptr(seed), _ptr(transpose_seed), amax.data_ptr(),
+                                       codes.data_ptr(), scales.data_ptr(), t.data_ptr(), codes_t.data_ptr(),
+                                       scales_t.data_ptr(), t_t.data_ptr(), m, k, _stream()), "vq_cast_nvfp4_pair")
+    return codes, scales, t, codes_t, scales_t, t_t
+
+
+@N.device_guarded
+def _cast_square(weight):
+    n, k = weight.shape
+    codes, scales, t = _matrix_outputs(n, k, weight.device)
+    codes_t, scales_t, _ = _matrix_outputs(k, n, weight.device)
+    amax = torch.empty((), dtype=torch.float32, device=weight.device)
+    N.check(N.lib().vq_cast_nvfp4_square(weight.data_ptr(), amax.data_ptr(), codes.data_ptr(), scales.data_ptr(),
+                                         codes_t.data_ptr(), scales_t.data_ptr(), t.data_ptr(), n, k, _stream()),
+            "vq_cast_nvfp4_square")
+    return codes, scales, codes_t, scales_t, t
 
 
 def quantize_nvfp4_square(weight: torch.Tensor):
@@ -235,6 +306,8 @@ def quantize_nvfp4_square(weight: torch.Tensor):
         raise NotImplementedError("quantize_nvfp4_square takes a bfloat16 matrix")
     n, k = weight.shape
     weight = weight.contiguous()
+    if _two_way(weight):
+        return _cast_square(weight)
     t = O.calculate_global_scale(weight, FP4_MAX, E4M3_MAX)
     amax = weight.abs().view(n // BLOCK_SIZE, BLOCK_SIZE, k // BLOCK_SIZE, BLOCK_SIZE).amax((1, 3))
     scale = torch.ops.quantized_ops.vmap((amax / FP4_MAX / t).clamp(max=E4M3_MAX),
