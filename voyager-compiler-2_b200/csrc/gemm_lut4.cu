@@ -11,37 +11,47 @@
 // (reference ops/quantized.py:574-591), the products are exact in float32 and the sum is float32:
 // the result differs from the operator's dequantize-then-matmul in summation order only.
 //
-// The kernel is bound by HBM (the weight bytes) and, next, by instruction issue (decoding a weight
-// is a table lookup and a multiply).  A CTA owns 256 weight rows x one K slice (1024, or 512 for small weights):
-//   * prologue: the activation slice is decoded into shared memory once (M x 1024 bfloat16, the
-//     four elements a lane needs per MMA step stored so that a warp's loads touch every bank once)
-//     and a 256-entry table maps a packed byte to its two codebook values as a bfloat16 pair --
-//     one copy per lane (32 random indices into a single table would collide on banks about
-//     3.5-fold), rows 256 bytes apart at a 64 KB-aligned shared address, because the lookups are
-//     what the loop does most and this makes a lookup three instructions: byte-permute (address),
-//     load, packed multiply (scale);
-//   * sixteen warps of 16 rows each stream the weight slice with 16-byte loads (32 weights per
-//     lane and load, two rows per lane in flight), look both nibbles of a byte up with one
-//     shared-memory load, scale them with one packed multiply and feed mma.sync m16n8k16 --
-//     M = 16 activation rows is exactly the instruction's height, the tensor-core form that fits a
-//     16-row problem (a 128-row tcgen05 tile would be 7/8 padding);
-//   * K slices are combined deterministically: every CTA writes its float32 partial tile to a
-//     workspace, and the last CTA of a row tile to arrive (a counter per tile) adds the partials in
-//     slice order, applies alpha and bias, rounds once and resets the counter.
+// The kernel is bound by HBM (the weight bytes) and, next, by shared-memory lookups and instruction
+// issue (decoding a weight is a table lookup and a multiply), so every SM streams the same share of the
+// weight from its first cycle to its last:
+//   * the weight is a flat list of (32-row tile, 128 weights of K) steps -- one list per K slice, as many
+//     slices as the decoded activations need to fit in shared memory (2048 of K for M <= 8, 1024 for 16 and 32
+//     rows) -- and the list is cut evenly over CTAs and then over a CTA's sixteen warps, wherever in a tile
+//     the cut falls;
+//   * each warp has a ring of two steps of its own in shared memory, filled by TMA (32 rows x 64 bytes, and 16 bytes
+//     of block scales per row), so the strided rows cost the load/store pipe, which the lookups need, nothing: loading
+//     them with 16-byte loads straight into registers held that pipe at 32 us for gate/up.  A step is read into
+//     registers at once and its slot refilled, across tiles; the first two are in flight before the prologue;
+//   * prologue: the activation slice is decoded into shared memory once (the four elements a lane needs per
+//     MMA step stored so that a warp's loads touch every bank once) and a 256-entry table maps a packed
+//     byte to its two codebook values as a bfloat16 pair -- one copy per lane (32 random indices into a
+//     single table would collide on banks about 3.5-fold), rows 256 bytes apart at a 64 KB-aligned shared
+//     address, which makes a lookup three instructions: byte-permute (address), load, packed multiply (scale);
+//   * the weights are the MMA's 16-row operand, so that up to 8 activation rows cost one MMA and one load per
+//     256 weights, and four rows of a lane share a load;
+//   * a tile that several warps of a CTA share is added up in shared memory, one that several CTAs share
+//     through a workspace by the last to arrive (a counter per tile), each in a fixed order.
+//
+// gate/up projection of Llama-3.1-8B (28672 x 4096, 62 MB): 24.8 us for one row (44 with CTAs of 256 rows x 1024
+// weights of K that each decoded the activations and met at a barrier per tile), 39 us for 16 rows (57 before);
+// down projection (4096 x 14336): 18.4 and 32 us (25 and 41 before).
+// What is left beside HBM (11 us for gate/up) is the latency of lookup, multiply and MMA at four warps a scheduler.
 
+#include <cuda.h>
 #include <cuda_bf16.h>
-#include <mma.h>
+#include <string.h>
 
+#include "sm100_ptx.cuh"
 #include "vq_common.cuh"
 
 namespace vq {
 namespace {
 
-constexpr int L4_ROWS_PER_WARP = 16;
+using namespace sm100;
+
 constexpr int L4_WARPS = 16;
-constexpr int L4_ROWS = L4_ROWS_PER_WARP * L4_WARPS;   // 256 weight rows per CTA
-constexpr int L4_KC = 1024;                            // longest K slice per CTA
 constexpr int L4_THREADS = 32 * L4_WARPS;
+constexpr int L4_STEP = 128;                           // weights of K per step and row
 // The byte table: one 256-byte row per byte value, lane l reading word l of the row.  It sits at
 // shared-memory address 0x10000, so that a lookup address is the lane's base address with its second
 // byte replaced by the packed byte -- one byte-permute instruction, no shift, mask or add.
@@ -65,12 +75,20 @@ struct Lut4Params {
   int alpha_dt;
   const void* bias;
   int bias_dt;
-  float* workspace;         // [k_slices][row_tiles][M_pad][128]
-  int* counters;            // [row_tiles], zero between launches
-  int k_slices, row_tiles;
-  int kc;                   // K slice length (a multiple of 128, at most L4_KC)
-  int a_after_table;        // the activation slice lies behind the table (two row tiles of activations)
+  float* workspace;         // [tiles][max_parts][accumulators of a tile]
+  int* counters;            // [tiles], zero between launches
+  int tiles;                // row tiles
+  int steps;                // K / L4_STEP
+  int slices;               // K slices: slice s holds steps s * steps / slices .. (s + 1) * steps / slices
+  int ctas;                 // CTAs per slice
+  int max_parts;            // workspace slots per tile
+  int lda_s;                // elements per activation row in shared memory
+  int bs_shift;
+  int small;                // every product of the cut's arithmetic fits 32 bits
+  int tma_scales;           // the scale rows are whole 16-byte pieces: map_s covers them
 };
+
+__device__ int g_lut4_error;
 
 __device__ __forceinline__ float lparam(const void* p, int64_t i, int dt) {
   if (dt == VQ_F32) return static_cast<const float*>(p)[i];
@@ -93,30 +111,97 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t v, uint32_t s) {
   return r;
 }
 
-// MT: 16-row activation tiles (1 or 2).
-template <int MT>
+// first step of slice `s` (the product is below 2^31: a slice is a few steps long)
+__host__ __device__ inline int l4_slice_begin(int s, int steps, int slices) { return (int)((uint32_t)s * (uint32_t)steps / (uint32_t)slices); }
+// part `i` of `n` equal parts of `total` begins here, and the part that holds step f.  `small`: total * n fits 32 bits
+// (64-bit divisions took half of a tile's finishing).
+__device__ inline int l4_cut(uint32_t i, uint32_t total, uint32_t n, bool small) {
+  return small ? (int)(i * total / n) : (int)((uint64_t)i * total / n);
+}
+__device__ inline int l4_part_of(uint32_t f, uint32_t total, uint32_t n, bool small) {
+  return small ? (int)(((f + 1) * n - 1) / total) : (int)(((uint64_t)(f + 1) * n - 1) / total);
+}
+
+// NT: activation rows in tiles of 8 (1..4).  RG: row groups of 8 per weight tile (4, or 2 beside many activation rows).
+template <int NT, int RG>
 __global__ void __launch_bounds__(L4_THREADS, 1)
-gemm_lut4_kernel(Lut4Params p) {
+gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s,
+                 const __grid_constant__ Lut4Params p) {
+  constexpr int TILE = 8 * RG;                  // weight rows per tile
+  constexpr int RT = RG / 2;                    // 16-row MMA tiles of it
+  constexpr int E = RT * NT * 4;                // accumulators per lane
   extern __shared__ __align__(16) uint8_t l4_smem[];
   // dynamic shared memory starts a little above the window's first kilobyte; the table is placed so that
-  // its shared address is exactly L4_TABLE_ADDR, the activation slice before it (or behind it when large)
+  // its shared address is exactly L4_TABLE_ADDR, the scale slots and the partial tiles before it, the activations
+  // and the weight ring behind it
   const uint32_t dyn_base = (uint32_t)__cvta_generic_to_shared(l4_smem);
   const uint32_t table_offset = L4_TABLE_ADDR - dyn_base;
-  uint32_t* table = reinterpret_cast<uint32_t*>(l4_smem + table_offset);           // [256][64 words], 32 used
-  __nv_bfloat16* sa = reinterpret_cast<__nv_bfloat16*>(
-      l4_smem + (p.a_after_table ? table_offset + L4_TABLE_BYTES : ((16u - (dyn_base & 15u)) & 15u)));   // [MT * 16][L4_KC + pad]
-  constexpr int SA_LD = L4_KC + L4_APAD;
-  __shared__ int s_last;
-  __shared__ float a_levels[256];                                                  // the activation's codebook
-
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t* table = reinterpret_cast<uint32_t*>(l4_smem + table_offset);           // [256][64 words], 32 used
+  uint8_t* slots = l4_smem + ((128u - (dyn_base & 127u)) & 127u) + warp * (2 * TILE * 16);   // this warp's [2][TILE][16]
+  float* heads = reinterpret_cast<float*>(l4_smem + ((128u - (dyn_base & 127u)) & 127u) + L4_WARPS * 2 * TILE * 16);   // [warps][E][32]
+  uint8_t* rings = l4_smem + table_offset + L4_TABLE_BYTES;                        // [warps][2][TILE][64]
+  uint8_t* ring = rings + warp * (2 * TILE * 64);
+  __nv_bfloat16* sa = reinterpret_cast<__nv_bfloat16*>(rings + L4_WARPS * 2 * TILE * 64);   // [NT * 8][lda_s]
+  // a warp's unfinished last tile lies in its own ring, which is empty by then
+  auto tails = [&](int w) { return reinterpret_cast<float*>(rings + w * (2 * TILE * 64)); };
+  __shared__ __align__(8) uint64_t bars[L4_WARPS][2];
+  __shared__ int s_abort;
+  volatile int* abort_flag = &s_abort;
+  __shared__ float a_levels[256];                                                  // the activation's codebook
+  __shared__ uint16_t w_levels[16];
+
   const int g = lane >> 2, t = lane & 3;
   const int slice = blockIdx.y;
-  const int k0 = slice * p.kc;
-  const int kc = min(p.kc, p.K - k0);                                              // a multiple of 128
+  const int step0 = l4_slice_begin(slice, p.steps, p.slices);
+  const int steps = l4_slice_begin(slice + 1, p.steps, p.slices) - step0;         // of K, per tile
+  const bool small = p.small != 0;
+  const int total = p.tiles * steps;
+  const int cta0 = l4_cut(blockIdx.x, total, p.ctas, small), cta1 = l4_cut(blockIdx.x + 1, total, p.ctas, small);
+  const int f0 = cta0 + l4_cut(warp, cta1 - cta0, L4_WARPS, small), f1 = cta0 + l4_cut(warp + 1, cta1 - cta0, L4_WARPS, small);
+
+  if (threadIdx.x < L4_WARPS * 2) mbar_init(&bars[0][0] + threadIdx.x, 1);
+  if (threadIdx.x == 0) s_abort = 0;
+  fence_barrier_init();
+  __syncthreads();
+
+  // ---- the weight stream of this warp ----
+  const int blocks_per_row = p.K >> p.bs_shift;
+  // 16 bytes of scales hold eight blocks; a step's blocks lie in one such piece
+  auto scale_piece = [&](int step) { return ((step0 + step) * L4_STEP) >> (p.bs_shift + 3); };
+  int ft = f0 / steps, fk = f0 - ft * steps;               // next step to fetch
+  int to_fetch = f1 - f0, fetch_slot = 1, fetched_piece = -1;
+  struct Scales { uint32_t s[RG]; };
+  auto fetch = [&](int stage, Scales& sc) {
+    if (to_fetch <= 0) return;
+    --to_fetch;
+    if (p.tma_scales) {
+      const int piece = scale_piece(fk);
+      const bool fresh = fk == 0 || piece != fetched_piece;
+      fetched_piece = piece;
+      if (fresh) fetch_slot ^= 1;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&bars[warp][stage], TILE * 64 + (fresh ? TILE * 16 : 0));
+        tma_load_3d(ring + stage * (TILE * 64), &map_w, &bars[warp][stage], (step0 + fk) * 64, ft * TILE, 0);
+        if (fresh) tma_load_3d(slots + fetch_slot * (TILE * 16), &map_s, &bars[warp][stage], piece * 8, ft * TILE, 0);
+      }
+    } else {
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&bars[warp][stage], TILE * 64);
+        tma_load_3d(ring + stage * (TILE * 64), &map_w, &bars[warp][stage], (step0 + fk) * 64, ft * TILE, 0);
+      }
+#pragma unroll
+      for (int j = 0; j < RG; ++j)   // rows past the end of the weight read row N - 1's scales; their results are never stored
+        sc.s[j] = __ldg(static_cast<const uint16_t*>(p.w_scale) + (int64_t)min(ft * TILE + 8 * j + g, p.N - 1) * blocks_per_row +
+                        (((step0 + fk) * L4_STEP + t * 32) >> p.bs_shift));
+    }
+    if (++fk == steps) { fk = 0; ++ft; }
+  };
+  Scales sc0, sc1;
+  fetch(0, sc0);
+  fetch(1, sc1);
 
   // ---- prologue: byte table and the decoded activation slice ----
-  __shared__ uint16_t w_levels[16];
   if (threadIdx.x < 16) w_levels[threadIdx.x] = static_cast<const uint16_t*>(p.w_levels)[threadIdx.x];
   if (p.a_levels != nullptr && (int)threadIdx.x < p.n_a_levels)
     a_levels[threadIdx.x] = __bfloat162float(static_cast<const __nv_bfloat16*>(p.a_levels)[threadIdx.x]);
@@ -129,9 +214,10 @@ gemm_lut4_kernel(Lut4Params p) {
     const __nv_bfloat16* A = static_cast<const __nv_bfloat16*>(p.a);
     const __nv_bfloat16* S = static_cast<const __nv_bfloat16*>(p.a_scale);
     const bool coded = p.a_levels != nullptr;
-    const int groups = kc >> 3;                                                    // 8 elements per thread and step
-    constexpr int BATCH = 8;                                                       // loads in flight per thread
-    for (int base = 0; base < MT * 16 * groups; base += BATCH * L4_THREADS) {
+    const int k0 = step0 * L4_STEP;
+    const int groups = steps * (L4_STEP / 8);                                      // 8 elements per thread and step
+    constexpr int BATCH = 4;                                                       // loads in flight per thread
+    for (int base = 0; base < NT * 8 * groups; base += BATCH * L4_THREADS) {
       uint4 raw[BATCH];
       float scl[BATCH];
 #pragma unroll
@@ -140,15 +226,15 @@ gemm_lut4_kernel(Lut4Params p) {
         const int m = idx / groups, kk = (idx - m * groups) << 3;
         raw[u] = make_uint4(0, 0, 0, 0);
         scl[u] = 1.0f;
-        if (idx < MT * 16 * groups && m < p.M) {
+        if (idx < NT * 8 * groups && m < p.M) {
           raw[u] = *reinterpret_cast<const uint4*>(A + (int64_t)m * p.lda + k0 + kk);
-          if (S) scl[u] = __bfloat162float(S[(int64_t)m * (p.K / p.bs) + (k0 + kk) / p.bs]);
+          if (S) scl[u] = __bfloat162float(S[(int64_t)m * blocks_per_row + ((k0 + kk) >> p.bs_shift)]);
         }
       }
 #pragma unroll
       for (int u = 0; u < BATCH; ++u) {
         const int idx = base + u * L4_THREADS + threadIdx.x;
-        if (idx >= MT * 16 * groups) continue;
+        if (idx >= NT * 8 * groups) continue;
         const int m = idx / groups, kk = (idx - m * groups) << 3;
         uint4 packed = raw[u];
         if (m < p.M && (S != nullptr || coded)) {
@@ -169,7 +255,7 @@ gemm_lut4_kernel(Lut4Params p) {
         // element 128 i + 32 t + 4 s + e of the slice lives at column 128 i + 16 s + 4 t + e: lane t of a warp
         // reads its four elements of step s eight bytes after lane t - 1's
         const int seg = kk & 127, tt = seg >> 5, ss = (seg & 31) >> 2;              // ss is even: steps ss and ss + 1
-        __nv_bfloat16* dst = sa + m * SA_LD + (kk & ~127) + 16 * ss + 4 * tt;
+        __nv_bfloat16* dst = sa + m * p.lda_s + (kk & ~127) + 16 * ss + 4 * tt;
         *reinterpret_cast<uint2*>(dst) = make_uint2(packed.x, packed.y);
         *reinterpret_cast<uint2*>(dst + 16) = make_uint2(packed.z, packed.w);
       }
@@ -177,132 +263,186 @@ gemm_lut4_kernel(Lut4Params p) {
   }
   __syncthreads();
 
-  // ---- main loop: this warp's 16 weight rows over the K slice, one row tile of the CTA after the other ----
-  for (int row_tile = blockIdx.x; row_tile < p.row_tiles; row_tile += gridDim.x) {
-  const int n_base = row_tile * L4_ROWS + warp * L4_ROWS_PER_WARP;
-  float acc[MT][2][4];
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[mt][j][e] = 0.0f;
-
   // This lane's column of the table as a 32-bit shared address; its second byte is zero.
   const uint32_t tb_lane = L4_TABLE_ADDR + 4u * lane;
-  const int row_bytes = p.K >> 1;
-  const int blocks_per_row = p.K / p.bs;
-  const int bs_shift = 31 - __clz(p.bs);                  // the block size is a power of two (32, 64, 128, ...)
-  // rows past the end of the weight read row N - 1 again (valid memory); their results are never stored
-  const uint8_t* wrow[2];
-  const uint16_t* srow[2];
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int n = min(n_base + 8 * j + g, p.N - 1);
-    wrow[j] = p.w + (int64_t)n * row_bytes + (k0 >> 1) + t * 16;
-    srow[j] = static_cast<const uint16_t*>(p.w_scale) + (int64_t)n * blocks_per_row + ((k0 + t * 32) >> bs_shift);
-  }
-  const int iters = kc >> 7;                              // 128 weights per row and iteration
-  const int scale_step_shift = 7 - bs_shift;              // blocks per iteration = 128 / bs (>= 0 for bs <= 128)
-
-  struct Vec { uint4 w[2]; uint32_t s[2]; };
-  auto fetch = [&](int it, Vec& v) {
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      v.w[j] = __ldcs(reinterpret_cast<const uint4*>(wrow[j] + it * 64));          // streamed once: evict first
-      const int blk = scale_step_shift >= 0 ? (it << scale_step_shift) : (it >> -scale_step_shift);
-      const uint32_t h = __ldg(srow[j] + blk);
-      v.s[j] = h | (h << 16);
-    }
-  };
   // the table entry of byte `which` (0..3) of `word`: address = tb_lane with byte 1 replaced by that byte
   auto lookup = [&](uint32_t word, int which) {
     uint32_t r;
     // not volatile: the table is constant once the CTA has passed its barrier, and the scheduler may then
-    // hoist an iteration's lookups ahead of the MMAs that consume them
+    // hoist a step's lookups ahead of the MMAs that consume them
     asm("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(__byte_perm(word, tb_lane, 0x7604u | ((uint32_t)which << 4))));
     return r;
   };
-  // the eight MMA steps of one iteration: step s takes bytes 2 s and 2 s + 1 of each row's 16-byte vector
-  auto compute = [&](int it, const Vec& v) {
-    const __nv_bfloat16* a_it = sa + it * 128 + t * 4;
+  float acc[RT][NT][4];
+  auto clear = [&]() {
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[r][n][e] = 0.0f;
+  };
+  // the eight MMAs deep contraction of one step: MMA s takes bytes 2 s and 2 s + 1 of each row's 16-byte vector, i.e.
+  // elements k = 32 t + 4 s + {0..3}, as its (k, k + 1) and (k + 8, k + 9) pairs
+  auto compute = [&](int k, const uint4 (&w8)[RG], const uint32_t (&sc)[RG]) {
+    const __nv_bfloat16* a_it = sa + g * p.lda_s + k * L4_STEP + t * 4;
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
-      uint32_t af[MT][4];   // rows g and g + 8 of every 16-row tile, elements k = 32 t + 4 s + {0..3}
+      uint2 af[NT];
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        const uint2 top = *reinterpret_cast<const uint2*>(a_it + (mt * 16 + g) * SA_LD + 16 * s);
-        const uint2 bot = *reinterpret_cast<const uint2*>(a_it + (mt * 16 + g + 8) * SA_LD + 16 * s);
-        af[mt][0] = top.x; af[mt][1] = bot.x; af[mt][2] = top.y; af[mt][3] = bot.y;
-      }
+      for (int n = 0; n < NT; ++n) af[n] = *reinterpret_cast<const uint2*>(a_it + n * 8 * p.lda_s + 16 * s);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const uint32_t word = s < 2 ? v.w[j].x : s < 4 ? v.w[j].y : s < 6 ? v.w[j].z : v.w[j].w;
-        const uint32_t b0 = mul_bf16x2(lookup(word, 2 * (s & 1)), v.s[j]);         // weights k, k + 1
-        const uint32_t b1 = mul_bf16x2(lookup(word, 2 * (s & 1) + 1), v.s[j]);     // weights k + 2, k + 3
+      for (int r = 0; r < RT; ++r) {
+        uint32_t b[2][2];
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) mma_bf16_16816(acc[mt][j], af[mt][0], af[mt][1], af[mt][2], af[mt][3], b0, b1);
+        for (int h = 0; h < 2; ++h) {
+          const uint4& w = w8[2 * r + h];
+          const uint32_t word = s < 2 ? w.x : s < 4 ? w.y : s < 6 ? w.z : w.w;
+          b[h][0] = mul_bf16x2(lookup(word, 2 * (s & 1)), sc[2 * r + h]);
+          b[h][1] = mul_bf16x2(lookup(word, 2 * (s & 1) + 1), sc[2 * r + h]);
+        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) mma_bf16_16816(acc[r][n], b[0][0], b[1][0], b[0][1], b[1][1], af[n].x, af[n].y);
       }
     }
   };
-  // three vector sets rotate by name, not by copy: two iterations' loads are always in flight
-  Vec va, vb, vc;
-  if (iters > 0) fetch(0, va);
-  if (iters > 1) fetch(1, vb);
-  int it = 0;
-  for (; it + 3 <= iters; it += 3) {
-    if (it + 2 < iters) fetch(it + 2, vc);
-    compute(it, va);
-    if (it + 3 < iters) fetch(it + 3, va);
-    compute(it + 1, vb);
-    if (it + 4 < iters) fetch(it + 4, vb);
-    compute(it + 2, vc);
-  }
-  if (it < iters) {
-    if (it + 2 < iters) fetch(it + 2, vc);
-    compute(it, va);
-    if (it + 1 < iters) compute(it + 1, vb);
-    if (it + 2 < iters) compute(it + 2, vc);
-  }
 
-  // ---- partial tile to the workspace: [slice][row_tile][m][128 columns] ----
-  // accumulator element e of group j: row m = g (+8 for e >= 2), column n = 8 j + 2 t + (e & 1)
-  const int m_pad = MT * 16;
-  float* part = p.workspace + ((int64_t)slice * p.row_tiles + row_tile) * m_pad * L4_ROWS;
+  // ---- the finished sum of one tile over this CTA's part of this slice ----
+  // accumulator e of MMA tile (r, n): weight row 16 r + g (+ 8 for e >= 2), activation row 8 n + 2 t + (e & 1)
+  auto output = [&](int tile) {
+    const float alpha = p.alpha ? lparam(p.alpha, 0, p.alpha_dt) : 1.0f;
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
+    for (int r = 0; r < RT; ++r)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int col = warp * L4_ROWS_PER_WARP + 8 * j + 2 * t;
-      *reinterpret_cast<float2*>(part + (mt * 16 + g) * L4_ROWS + col) = make_float2(acc[mt][j][0], acc[mt][j][1]);
-      *reinterpret_cast<float2*>(part + (mt * 16 + g + 8) * L4_ROWS + col) = make_float2(acc[mt][j][2], acc[mt][j][3]);
+      for (int h = 0; h < 2; ++h) {
+        const int row = tile * TILE + 16 * r + 8 * h + g;
+        if (row >= p.N) continue;
+        const float bias = p.bias ? lparam(p.bias, row, p.bias_dt) : 0.0f;
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int m = 8 * n + 2 * t + e;
+            if (m >= p.M) continue;
+            float sum = acc[r][n][2 * h + e];
+            if (p.alpha) sum = __fmul_rn(sum, alpha);
+            if (p.bias) sum = __fadd_rn(sum, bias);
+            const int64_t o = (int64_t)m * p.N + row;
+            if (p.out_dt == VQ_F32) static_cast<float*>(p.out)[o] = sum;
+            else if (p.out_dt == VQ_BF16) static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(sum);
+            else static_cast<__half*>(p.out)[o] = __float2half_rn(sum);
+          }
+      }
+  };
+  auto finish = [&](int tile) {
+    // the parts of this tile, over all slices and CTAs; mine is number `mine`
+    int parts = 0, mine = 0;
+    for (int s = lane; s < p.slices; s += 32) {
+      const int n = l4_slice_begin(s + 1, p.steps, p.slices) - l4_slice_begin(s, p.steps, p.slices);
+      const int first = l4_part_of(tile * n, p.tiles * n, p.ctas, small);
+      const int last = l4_part_of((tile + 1) * n - 1, p.tiles * n, p.ctas, small);
+      parts += last - first + 1;
+      if (s < slice) mine += last - first + 1;
+      if (s == slice) mine += blockIdx.x - first;
     }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&p.counters[row_tile], 1) == p.k_slices - 1;
-  __syncthreads();
-  const bool last = s_last != 0;
-  __syncthreads();   // s_last is rewritten for the CTA's next row tile
-  if (!last) continue;
-  __threadfence();
+    parts = __reduce_add_sync(0xFFFFFFFFu, parts);
+    mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+    if (parts > 1) {
+      float* slots = p.workspace + (int64_t)tile * p.max_parts * (E * 32) + lane;
+      float* my = slots + (int64_t)mine * (E * 32);
+#pragma unroll
+      for (int e = 0; e < E; ++e) __stcg(my + e * 32, acc[e / (NT * 4)][(e / 4) % NT][e % 4]);
+      __threadfence();
+      __syncwarp();
+      int last = 0;
+      if (lane == 0) last = atomicAdd(&p.counters[tile], 1) == parts - 1;
+      if (!__shfl_sync(0xFFFFFFFFu, last, 0)) return;
+      __threadfence();
+      clear();
+      for (int q = 0; q < parts; ++q)
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[e / (NT * 4)][(e / 4) % NT][e % 4] += __ldcg(slots + (int64_t)q * (E * 32) + e * 32);
+      if (lane == 0) p.counters[tile] = 0;   // ready for the next launch
+    }
+    output(tile);
+  };
 
-  // ---- the last CTA of the row tile adds the slices in order and writes the output ----
-  const float alpha = p.alpha ? lparam(p.alpha, 0, p.alpha_dt) : 1.0f;
-  for (int idx = threadIdx.x; idx < p.M * L4_ROWS; idx += L4_THREADS) {
-    const int m = idx / L4_ROWS, c = idx - m * L4_ROWS;
-    const int n = row_tile * L4_ROWS + c;
-    if (n >= p.N) continue;
-    float sum = 0.0f;
-    for (int sl = 0; sl < p.k_slices; ++sl)
-      sum += __ldcg(p.workspace + (((int64_t)sl * p.row_tiles + row_tile) * m_pad + m) * L4_ROWS + c);
-    if (p.alpha) sum = __fmul_rn(sum, alpha);
-    if (p.bias) sum = __fadd_rn(sum, lparam(p.bias, n, p.bias_dt));
-    const int64_t o = (int64_t)m * p.N + n;
-    if (p.out_dt == VQ_F32) static_cast<float*>(p.out)[o] = sum;
-    else if (p.out_dt == VQ_BF16) static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(sum);
-    else static_cast<__half*>(p.out)[o] = __float2half_rn(sum);
+  // ---- main loop ----
+  clear();
+  int ct = f0 / steps, ck = f0 - ct * steps;
+  bool whole = ck == 0;                          // this warp has the tile from its first step
+  int left = f1 - f0, read_slot = 1, read_piece = -1;
+  uint32_t phase = 0;
+  auto step = [&](int stage, Scales& next) {
+    if (!__all_sync(0xFFFFFFFFu, mbar_wait(&bars[warp][stage], phase, abort_flag))) return false;
+    uint4 w8[RG];
+    uint32_t sc[RG];
+#pragma unroll
+    for (int j = 0; j < RG; ++j)
+      w8[j] = *reinterpret_cast<const uint4*>(ring + stage * (TILE * 64) + (8 * j + g) * 64 + t * 16);
+    if (p.tma_scales) {
+      const int piece = scale_piece(ck);
+      if (ck == 0 || piece != read_piece) read_slot ^= 1;
+      read_piece = piece;
+      const int blk = (((step0 + ck) * L4_STEP + t * 32) >> p.bs_shift) & 7;
+#pragma unroll
+      for (int j = 0; j < RG; ++j)
+        sc[j] = *reinterpret_cast<const uint16_t*>(slots + read_slot * (TILE * 16) + (8 * j + g) * 16 + blk * 2) * 0x10001u;
+    } else {
+#pragma unroll
+      for (int j = 0; j < RG; ++j) sc[j] = next.s[j] * 0x10001u;
+    }
+    __syncwarp();   // the step is in registers: its slot may be refilled
+    fetch(stage, next);
+    compute(ck, w8, sc);
+    --left;
+    if (++ck == steps || left == 0) {
+      if (whole && ck == steps) {
+        finish(ct);
+      } else {
+        float* slot = (whole ? tails(warp) : heads + warp * (E * 32)) + lane;
+#pragma unroll
+        for (int e = 0; e < E; ++e) slot[e * 32] = acc[e / (NT * 4)][(e / 4) % NT][e % 4];
+      }
+      clear();
+      whole = true;
+      ck = 0;
+      ++ct;
+    }
+    return true;
+  };
+  bool ok = true;
+  while (left > 0) {
+    if (!(ok = step(0, sc0))) break;
+    if (left > 0 && !(ok = step(1, sc1))) break;
+    phase ^= 1;
   }
-  if (threadIdx.x == 0) p.counters[row_tile] = 0;   // ready for the next launch
+  if (!ok) {   // a load never arrived: let what is in flight end (waiting again with a limit) and report it
+    for (int i = 0; i < 2; ++i)
+      for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(&bars[warp][i], phase); ++spin) {}
+    if (lane == 0) atomicExch(&g_lut4_error, VQ_ETIMEOUT);
+  }
+  __syncthreads();
+
+  // ---- tiles that several warps, or this CTA's first or last warp and another CTA, share ----
+  if (cta0 == cta1 || *abort_flag) return;
+  const int len = cta1 - cta0;
+  const int tile_first = cta0 / steps, tile_last = (cta1 - 1) / steps;
+  for (int tile = tile_first + warp; tile <= tile_last; tile += L4_WARPS) {
+    const int b = tile * steps, e = b + steps;
+    const int lo = max(b, cta0), hi = min(e, cta1);
+    int w = l4_part_of(lo - cta0, len, L4_WARPS, small);
+    if (cta0 + l4_cut(w, len, L4_WARPS, small) <= b && cta0 + l4_cut(w + 1, len, L4_WARPS, small) >= e) continue;   // one warp had it all
+    const int w_last = l4_part_of(hi - 1 - cta0, len, L4_WARPS, small);
+    clear();
+    for (; w <= w_last; ++w) {
+      const int begin = cta0 + l4_cut(w, len, L4_WARPS, small);
+      if (begin == cta0 + l4_cut(w + 1, len, L4_WARPS, small)) continue;   // a warp without steps
+      const float* slot = (begin <= b ? tails(w) : heads + w * (E * 32)) + lane;
+#pragma unroll
+      for (int q = 0; q < E; ++q) acc[q / (NT * 4)][(q / 4) % NT][q % 4] += slot[q * 32];
+    }
+    finish(tile);
   }
 }
 
@@ -322,23 +462,83 @@ __global__ void pack_lut4_kernel(const __nv_bfloat16* __restrict__ codes, uint8_
 
 using namespace vq;
 
+// Boxes of box_x elements x box_rows rows of a dense [rows, cols] matrix, unswizzled (eight lanes read 128 neighbouring
+// bytes); rows past the end arrive as zeros.
+static int lut4_map(CUtensorMap* map, const void* base, CUtensorMapDataType type, int elem, int64_t cols, int64_t rows,
+                    int box_x, int box_rows) {
+  typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static EncodeFn enc = nullptr;
+  if (!enc) {
+    void* sym = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      return fail(VQ_ECUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    enc = reinterpret_cast<EncodeFn>(sym);
+  }
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 1};
+  const cuuint64_t strides[2] = {(cuuint64_t)(cols * elem), (cuuint64_t)(cols * elem * rows)};
+  const cuuint32_t box[3] = {(cuuint32_t)box_x, (cuuint32_t)box_rows, 1}, unit[3] = {1, 1, 1};
+  const CUresult r = enc(map, type, 3, const_cast<void*>(base), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(VQ_ECUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+  return VQ_OK;
+}
+
+// whether a launch gave up waiting for a load (read by vq_gemm_status)
+namespace vq {
+int lut4_status(int reset) {
+  int value = 0;
+  if (cudaMemcpyFromSymbol(&value, g_lut4_error, sizeof(int)) != cudaSuccess) return VQ_ECUDA;
+  if (reset && value) {
+    const int zero = 0;
+    cudaMemcpyToSymbol(g_lut4_error, &zero, sizeof(int));
+  }
+  return value;
+}
+}  // namespace vq
+
 extern "C" {
 
-// K slice length: 1024, or 512 when the weight has too few 256-row tiles to give every SM a CTA
-static int lut4_slice_length(int64_t N, int64_t K) {
-  const int64_t tiles = (N + L4_ROWS - 1) / L4_ROWS;
-  return tiles * ((K + L4_KC - 1) / L4_KC) < kSmCount && K > 512 ? 512 : L4_KC;
+// How a product is cut: 8 * NT activation rows, weight tiles of 8 * RG rows, K slices, CTAs per slice.
+struct Lut4Plan {
+  int nt, rg, tiles, steps, slices, ctas, max_parts, lda_s;
+};
+static Lut4Plan lut4_plan(int64_t M, int64_t N, int64_t K) {
+  Lut4Plan q{};
+  q.nt = (int)((M + 7) / 8);
+  q.rg = q.nt <= 2 ? 4 : 2;                                  // partial tiles of both sets beside the activations
+  q.tiles = (int)((N + 8 * q.rg - 1) / (8 * q.rg));
+  q.steps = (int)(K / L4_STEP);
+  static const int longest[5] = {0, 16, 8, 10, 8};           // steps of activations that fit behind table and ring
+  const int least_slices = (q.steps + longest[q.nt] - 1) / longest[q.nt];
+  // as few slices as that allows, or up to a quarter more where they use more of the SMs
+  q.slices = least_slices;
+  for (int n = least_slices + 1; n <= least_slices + least_slices / 4 && n <= kSmCount; ++n)
+    if (kSmCount / n * n > kSmCount / q.slices * q.slices) q.slices = n;
+  // one CTA per SM; a small weight has a step for each warp of a CTA at least
+  const int64_t total = (int64_t)q.tiles * (q.steps / q.slices);
+  int64_t ctas = kSmCount / q.slices, most = (total + L4_WARPS - 1) / L4_WARPS;
+  if (ctas > most) ctas = most;
+  q.ctas = ctas < 1 ? 1 : (int)ctas;
+  const int slice_max = (q.steps + q.slices - 1) / q.slices;
+  q.lda_s = slice_max * L4_STEP + L4_APAD;
+  // a CTA has at least floor(total / ctas) consecutive steps of a slice, and a slice at most slice_max of a tile
+  const int64_t least = total / q.ctas < 1 ? 1 : total / q.ctas;
+  const int64_t per_slice = (slice_max - 1) / least + 2;
+  q.max_parts = (int)(q.slices * (per_slice < q.ctas ? per_slice : q.ctas));
+  return q;
 }
 
 int64_t vq_gemm_lut4_workspace_floats(int64_t M, int64_t N, int64_t K) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const int64_t m_pad = M <= 16 ? 16 : 32;
-  const int64_t kc = lut4_slice_length(N, K);
-  const int64_t slices = (K + kc - 1) / kc, tiles = (N + L4_ROWS - 1) / L4_ROWS;
-  return slices * tiles * m_pad * L4_ROWS;
+  if (M <= 0 || N <= 0 || K <= 0 || M > 32 || K % L4_STEP) return 0;
+  const Lut4Plan q = lut4_plan(M, N, K);
+  return (int64_t)q.tiles * q.max_parts * (q.nt * 8) * (q.rg * 8);
 }
 
-int64_t vq_gemm_lut4_counters(int64_t N) { return N <= 0 ? 0 : (N + L4_ROWS - 1) / L4_ROWS; }
+int64_t vq_gemm_lut4_counters(int64_t N) { return N <= 0 ? 0 : (N + 15) / 16; }
 
 int vq_pack_lut4(const void* codes, void* packed, int64_t rows, int64_t K, int* bad, void* stream) {
   VQ_REQUIRE(rows >= 0 && K >= 0 && K % 2 == 0, "vq_pack_lut4: K must be even");
@@ -375,31 +575,39 @@ int vq_gemm_lut4(const void* a, int64_t lda, const void* a_scale, const void* a_
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.bs = block_size; p.lda = lda;
   p.alpha = alpha; p.alpha_dt = alpha_dtype; p.bias = bias; p.bias_dt = bias_dtype;
   p.workspace = workspace; p.counters = counters;
-  p.kc = lut4_slice_length(N, K);
-  p.k_slices = (int)((K + p.kc - 1) / p.kc);
-  p.row_tiles = (int)((N + L4_ROWS - 1) / L4_ROWS);
-  VQ_REQUIRE(p.k_slices <= 65535, "vq_gemm_lut4: K too large");
-  const int mt = M <= 16 ? 1 : 2;
+  const Lut4Plan q = lut4_plan(M, N, K);
+  p.tiles = q.tiles; p.steps = q.steps; p.slices = q.slices; p.ctas = q.ctas; p.max_parts = q.max_parts; p.lda_s = q.lda_s;
+  while ((1 << p.bs_shift) < block_size) ++p.bs_shift;
+  VQ_REQUIRE(p.slices <= 65535 && (int64_t)q.tiles * q.steps < (1ll << 31), "vq_gemm_lut4: weight too large");
+  const int64_t most_ctas = q.ctas > L4_WARPS ? q.ctas : L4_WARPS;
+  p.small = ((int64_t)q.tiles * q.steps + 1) * most_ctas < (1ll << 32);
   // Shared memory: the table must sit at shared address L4_TABLE_ADDR.  Dynamic memory starts somewhere in
   // [1 KB, 4 KB) of the window (system + static variables), so reserving up to the table's end measured from
-  // 1 KB always suffices; one row tile of activations (33 KB) fits before the table, two go behind it.
-  const int a_bytes = mt * 16 * (L4_KC + L4_APAD) * (int)sizeof(__nv_bfloat16);
-  p.a_after_table = mt == 2;
-  const size_t smem = (size_t)L4_TABLE_ADDR + L4_TABLE_BYTES - 1024 + (p.a_after_table ? a_bytes : 0);
+  // 1 KB always suffices; scale slots and partial tiles (16 + 32 KB at most) fit before the table.
+  const int tile = q.rg * 8;
+  const int a_bytes = q.nt * 8 * q.lda_s * (int)sizeof(__nv_bfloat16);
+  const size_t smem = (size_t)L4_TABLE_ADDR + L4_TABLE_BYTES - 1024 + a_bytes + L4_WARPS * 2 * tile * 64;
+  constexpr int kMostSmem = (int)L4_TABLE_ADDR + L4_TABLE_BYTES - 1024 + 99328;   // 32 rows of 1040 elements + 32 KB
+  VQ_REQUIRE((int)smem <= kMostSmem, "vq_gemm_lut4: internal error: %d bytes of shared memory", (int)smem);
+  CUtensorMap map_w, map_s;
+  if (int e = lut4_map(&map_w, w_packed, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 2, N, 64, tile)) return e;
+  memset(&map_s, 0, sizeof(map_s));
+  p.tma_scales = (K / block_size) % 8 == 0 && (reinterpret_cast<uintptr_t>(w_scale) & 15) == 0;
+  if (p.tma_scales)
+    if (int e = lut4_map(&map_s, w_scale, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, K / block_size, N, 8, tile)) return e;
   static unsigned long long configured = 0;
   if (first_call_on_device(&configured)) {
-    cudaFuncSetAttribute(gemm_lut4_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)L4_TABLE_ADDR + L4_TABLE_BYTES - 1024);
-    cudaFuncSetAttribute(gemm_lut4_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)L4_TABLE_ADDR + L4_TABLE_BYTES - 1024 + 32 * (L4_KC + L4_APAD) * 2);
+    cudaFuncSetAttribute(gemm_lut4_kernel<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
+    cudaFuncSetAttribute(gemm_lut4_kernel<2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
+    cudaFuncSetAttribute(gemm_lut4_kernel<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
+    cudaFuncSetAttribute(gemm_lut4_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
   }
-  // about two CTAs' worth of row tiles per SM in all; with many row tiles a CTA takes several of them, one
-  // after the other, and decodes its activation slice once
-  const int per_slice = (2 * kSmCount + p.k_slices - 1) / p.k_slices;
-  dim3 grid((unsigned)(p.row_tiles < per_slice ? p.row_tiles : per_slice), (unsigned)p.k_slices);
+  const dim3 grid((unsigned)q.ctas, (unsigned)q.slices);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (mt == 1) gemm_lut4_kernel<1><<<grid, L4_THREADS, smem, st>>>(p);
-  else gemm_lut4_kernel<2><<<grid, L4_THREADS, smem, st>>>(p);
+  if (q.nt == 1) gemm_lut4_kernel<1, 4><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
+  else if (q.nt == 2) gemm_lut4_kernel<2, 4><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
+  else if (q.nt == 3) gemm_lut4_kernel<3, 2><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
+  else gemm_lut4_kernel<4, 2><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
   return check_launch("gemm_lut4_kernel");
 }
 

@@ -2416,6 +2416,7 @@ int vq_gemm_status(int reset) {
     cudaMemcpyToSymbol(g_gemm_error, &zero, sizeof(int));
   }
   if (value != 0) return fail(value, "a tensor-core GEMM gave up waiting on a barrier");
+  if (int lut4 = lut4_status(reset)) return fail(lut4, "a packed decode linear gave up waiting for a load");
   return VQ_OK;
 }
 

@@ -25,6 +25,8 @@ int check_launch(const char* what);
     if (!(cond)) return vq::fail(VQ_EINVAL, __VA_ARGS__); \
   } while (0)
 
+int lut4_status(int reset);   // gemm_lut4.cu
+
 constexpr int kSmCount = 148;
 
 // Per-device one-time set-up (function attributes such as the dynamic shared-memory limit
