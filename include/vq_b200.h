@@ -631,6 +631,16 @@ int vq_gemm_lut4(const void* a, int64_t lda, const void* a_scale, const void* a_
                  int out_dtype, int64_t N, int64_t K, const void* alpha, int alpha_dtype, const void* bias,
                  int bias_dtype, float* workspace, int* counters, void* stream);
 
+/* linear_mx (ops/quantized.py:662-723) for at most 32 activation rows on the operator's own storage: a [M, K] and w
+ * [N, K] bfloat16 codes with bfloat16 scales per `block_size` elements of K ([M, K / bs], [N, K / bs]); a_levels / w_levels:
+ * bfloat16 codebooks (w_levels 16 entries) or null when the codes are the values.  K is a multiple of 32 and of the
+ * block size (a power of two, 8 or more).  workspace: vq_gemm_mx_rows_workspace_bytes(M, N, K) bytes. */
+int64_t vq_gemm_mx_rows_workspace_bytes(int64_t M, int64_t N, int64_t K);
+int vq_gemm_mx_rows(const void* a, const void* a_scale, const void* a_levels, int n_a_levels, const void* w,
+                    const void* w_scale, const void* w_levels, int64_t block_size, void* out, int out_dtype, int64_t M,
+                    int64_t N, int64_t K, const void* alpha, int alpha_dtype, const void* bias, int bias_dtype,
+                    void* workspace, void* stream);
+
 /* Packs bfloat16-valued codebook indices codes [rows, K] (each 0..15, what quantize_mx returns
  * for a lookup format with an index table, quantize_pt2e.py:754-791) into vq_gemm_lut4's
  * w_packed layout.  *bad (device int, zeroed by the caller) is set if a value is not such an index. */

@@ -134,6 +134,8 @@ SIGNATURES = {
     "vq_cast_nvfp4": [_P, _P, _I, _P, _P, _P, _I64, _I64, _P],
     "vq_cast_nvfp4_pair": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _P],
     "vq_cast_nvfp4_square": [_P, _P, _P, _P, _P, _P, _P, _I64, _I64, _P],
+    "vq_gemm_mx_rows_workspace_bytes": [_I64, _I64, _I64],
+    "vq_gemm_mx_rows": [_P, _P, _P, _I, _P, _P, _P, _I64, _P, _I, _I64, _I64, _I64, _P, _I, _P, _I, _P, _P],
     "vq_kivi_read_2bit": [_P, _P, _P, _P, _I64, _I64, _I64, _I, _I64, _P],
     "vq_gptq_block": [_P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I, _F, _F, _I, ctypes.POINTER(VqRound),
                       ctypes.POINTER(VqRound), _P],
@@ -160,7 +162,7 @@ SIGNATURES = {
 }
 IN_BF16, IN_F16, IN_E4M3, IN_E5M2 = range(4)
 _INT64_RESULTS = ("vq_nvfp4_scale_bytes", "vq_rmsnorm_backward_programs", "vq_gemm_lut4_workspace_floats",
-                  "vq_gemm_lut4_counters")
+                  "vq_gemm_lut4_counters", "vq_gemm_mx_rows_workspace_bytes")
 
 
 def sources():

@@ -29,8 +29,13 @@
 //     address, which makes a lookup three instructions: byte-permute (address), load, packed multiply (scale);
 //   * the weights are the MMA's 16-row operand, so that up to 8 activation rows cost one MMA and one load per
 //     256 weights, and four rows of a lane share a load;
+//   * weights in the operator's own storage (bfloat16-valued codes, 2 bytes each: WIDE) stream the same way, 32 of K
+//     per step; their codes are the values themselves or indices that the same table decodes in pairs;
 //   * a tile that several warps of a CTA share is added up in shared memory, one that several CTAs share
 //     through a workspace by the last to arrive (a counter per tile), each in a fixed order.
+//
+// 4096 x 4096 from bfloat16 codes with blocks of 16, 7 rows (34 MB): 18.6 us; the tensor-core GEMM's 256-row tiles
+// gave 16 CTA pairs work for 68 us.
 //
 // gate/up projection of Llama-3.1-8B (28672 x 4096, 62 MB): 24.8 us for one row (44 with CTAs of 256 rows x 1024
 // weights of K that each decoded the activations and met at a barrier per tile), 39 us for 16 rows (57 before);
@@ -51,7 +56,8 @@ using namespace sm100;
 
 constexpr int L4_WARPS = 16;
 constexpr int L4_THREADS = 32 * L4_WARPS;
-constexpr int L4_STEP = 128;                           // weights of K per step and row
+// weights of K per step and row: 64 bytes
+template <bool WIDE> struct L4Step { static constexpr int value = WIDE ? 32 : 128; };
 // The byte table: one 256-byte row per byte value, lane l reading word l of the row.  It sits at
 // shared-memory address 0x10000, so that a lookup address is the lane's base address with its second
 // byte replaced by the packed byte -- one byte-permute instruction, no shift, mask or add.
@@ -64,9 +70,9 @@ struct Lut4Params {
   const void* a_scale;      // [M, K / bs] bfloat16 or null
   const void* a_levels;     // [n_a_levels] bfloat16 or null
   int n_a_levels;
-  const uint8_t* w;         // [N, K / 2]
+  const uint8_t* w;         // packed: [N, K / 2]
   const void* w_scale;      // [N, K / bs] bfloat16
-  const void* w_levels;     // [16] bfloat16
+  const void* w_levels;     // [16] bfloat16; wide codes: null when the codes are the values
   void* out;
   int out_dt;
   int M, N, K, bs;
@@ -78,7 +84,7 @@ struct Lut4Params {
   float* workspace;         // [tiles][max_parts][accumulators of a tile]
   int* counters;            // [tiles], zero between launches
   int tiles;                // row tiles
-  int steps;                // K / L4_STEP
+  int steps;                // K / step
   int slices;               // K slices: slice s holds steps s * steps / slices .. (s + 1) * steps / slices
   int ctas;                 // CTAs per slice
   int max_parts;            // workspace slots per tile
@@ -122,11 +128,33 @@ __device__ inline int l4_part_of(uint32_t f, uint32_t total, uint32_t n, bool sm
   return small ? (int)(((f + 1) * n - 1) / total) : (int)(((uint64_t)(f + 1) * n - 1) / total);
 }
 
+// One code's codebook entry as the generic read-back indexes it (truncate, wrap a negative once, clamp).
+__device__ __forceinline__ int code_index(float v, int n) {
+  long long i = (long long)v;
+  i = i < 0 ? i + n : i;
+  return (int)(i < 0 ? 0 : (i >= n ? n - 1 : i));
+}
+// a vector of wide codes with something other than 0..15 in it
+__device__ __noinline__ uint4 decode_odd(uint4 raw, const __nv_bfloat16* __restrict__ levels, uint32_t scale2) {
+  const float s = __uint_as_float(scale2 << 16);
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float a = __bfloat162float(levels[code_index(__uint_as_float(w[j] << 16), 16)]);
+    const float b = __bfloat162float(levels[code_index(__uint_as_float(w[j] & 0xFFFF0000u), 16)]);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(__fmul_rn(a, s), __fmul_rn(b, s));
+    o[j] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // NT: activation rows in tiles of 8 (1..4).  RG: row groups of 8 per weight tile (4, or 2 beside many activation rows).
-template <int NT, int RG>
+template <bool WIDE, int NT, int RG>
 __global__ void __launch_bounds__(L4_THREADS, 1)
 gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s,
                  const __grid_constant__ Lut4Params p) {
+  constexpr int L4_STEP = L4Step<WIDE>::value;
   constexpr int TILE = 8 * RG;                  // weight rows per tile
   constexpr int RT = RG / 2;                    // 16-row MMA tiles of it
   constexpr int E = RT * NT * 4;                // accumulators per lane
@@ -193,7 +221,7 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
       for (int j = 0; j < RG; ++j)   // rows past the end of the weight read row N - 1's scales; their results are never stored
         sc.s[j] = __ldg(static_cast<const uint16_t*>(p.w_scale) + (int64_t)min(ft * TILE + 8 * j + g, p.N - 1) * blocks_per_row +
-                        (((step0 + fk) * L4_STEP + t * 32) >> p.bs_shift));
+                        (((step0 + fk) * L4_STEP + t * (L4_STEP / 4)) >> p.bs_shift));
     }
     if (++fk == steps) { fk = 0; ++ft; }
   };
@@ -202,11 +230,11 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   fetch(1, sc1);
 
   // ---- prologue: byte table and the decoded activation slice ----
-  if (threadIdx.x < 16) w_levels[threadIdx.x] = static_cast<const uint16_t*>(p.w_levels)[threadIdx.x];
+  if (threadIdx.x < 16 && p.w_levels) w_levels[threadIdx.x] = static_cast<const uint16_t*>(p.w_levels)[threadIdx.x];
   if (p.a_levels != nullptr && (int)threadIdx.x < p.n_a_levels)
     a_levels[threadIdx.x] = __bfloat162float(static_cast<const __nv_bfloat16*>(p.a_levels)[threadIdx.x]);
   __syncthreads();
-  for (int i = threadIdx.x; i < 256 * 32; i += L4_THREADS) {
+  for (int i = threadIdx.x; i < 256 * 32 && p.w_levels; i += L4_THREADS) {
     const int byte = i >> 5;
     table[byte * 64 + (i & 31)] = (uint32_t)w_levels[byte & 15] | ((uint32_t)w_levels[byte >> 4] << 16);   // even element low
   }
@@ -243,7 +271,10 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             float v0 = __uint_as_float(w4[q] << 16), v1 = __uint_as_float(w4[q] & 0xFFFF0000u);
-            if (coded) {   // indices are exact small integers in bfloat16
+            if (coded && WIDE) {
+              v0 = a_levels[code_index(v0, p.n_a_levels)];
+              v1 = a_levels[code_index(v1, p.n_a_levels)];
+            } else if (coded) {   // indices are exact small integers in bfloat16
               v0 = a_levels[min(max((int)v0, 0), p.n_a_levels - 1)];
               v1 = a_levels[min(max((int)v1, 0), p.n_a_levels - 1)];
             }
@@ -251,6 +282,10 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             o4[q] = *reinterpret_cast<const uint32_t*>(&h);
           }
           packed = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+        }
+        if (WIDE) {   // a lane takes eight neighbouring elements of a step: they stay in order
+          *reinterpret_cast<uint4*>(sa + m * p.lda_s + kk) = packed;
+          continue;
         }
         // element 128 i + 32 t + 4 s + e of the slice lives at column 128 i + 16 s + 4 t + e: lane t of a warp
         // reads its four elements of step s eight bytes after lane t - 1's
@@ -305,6 +340,42 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         for (int n = 0; n < NT; ++n) mma_bf16_16816(acc[r][n], b[0][0], b[1][0], b[0][1], b[1][1], af[n].x, af[n].y);
       }
     }
+  };
+
+  // One step of wide codes: lane t has elements k = 8 t + {0..7} of each row, the first four for one MMA and the last
+  // four for another, as their (k, k + 1) and (k + 8, k + 9) pairs.
+  auto compute_wide = [&](int k, const uint4 (&w8)[RG], const uint32_t (&sc)[RG]) {
+    uint4 af[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+      af[n] = *reinterpret_cast<const uint4*>(sa + (n * 8 + g) * p.lda_s + k * L4_STEP + t * 8);
+    uint4 b[RG];
+#pragma unroll
+    for (int j = 0; j < RG; ++j) {
+      uint32_t w[4] = {w8[j].x, w8[j].y, w8[j].z, w8[j].w};
+      uint32_t odd = 0;
+      if (p.w_levels) {
+        const __nv_bfloat162 bias2 = __float2bfloat162_rn(128.0f);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          // 128 + code leaves an index in the low bits of each half, exactly for 0..15
+          const __nv_bfloat162 c = __hadd2_rn(*reinterpret_cast<const __nv_bfloat162*>(&w[q]), bias2);
+          const __nv_bfloat162 back = __hsub2_rn(c, bias2);
+          const uint32_t cb = *reinterpret_cast<const uint32_t*>(&c);
+          odd |= ((cb ^ 0x43004300u) & 0xFFF0FFF0u) | (*reinterpret_cast<const uint32_t*>(&back) ^ w[q]);
+          w[q] = lookup((cb & 0xFu) | ((cb >> 12) & 0xF0u), 0);
+        }
+      }
+      b[j] = make_uint4(mul_bf16x2(w[0], sc[j]), mul_bf16x2(w[1], sc[j]), mul_bf16x2(w[2], sc[j]), mul_bf16x2(w[3], sc[j]));
+      if (odd) b[j] = decode_odd(w8[j], static_cast<const __nv_bfloat16*>(p.w_levels), sc[j]);
+    }
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        mma_bf16_16816(acc[r][n], b[2 * r].x, b[2 * r + 1].x, b[2 * r].y, b[2 * r + 1].y, af[n].x, af[n].y);
+        mma_bf16_16816(acc[r][n], b[2 * r].z, b[2 * r + 1].z, b[2 * r].w, b[2 * r + 1].w, af[n].z, af[n].w);
+      }
   };
 
   // ---- the finished sum of one tile over this CTA's part of this slice ----
@@ -384,7 +455,7 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       const int piece = scale_piece(ck);
       if (ck == 0 || piece != read_piece) read_slot ^= 1;
       read_piece = piece;
-      const int blk = (((step0 + ck) * L4_STEP + t * 32) >> p.bs_shift) & 7;
+      const int blk = (((step0 + ck) * L4_STEP + t * (L4_STEP / 4)) >> p.bs_shift) & 7;
 #pragma unroll
       for (int j = 0; j < RG; ++j)
         sc[j] = *reinterpret_cast<const uint16_t*>(slots + read_slot * (TILE * 16) + (8 * j + g) * 16 + blk * 2) * 0x10001u;
@@ -394,7 +465,8 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
     __syncwarp();   // the step is in registers: its slot may be refilled
     fetch(stage, next);
-    compute(ck, w8, sc);
+    if constexpr (WIDE) compute_wide(ck, w8, sc);
+    else compute(ck, w8, sc);
     --left;
     if (++ck == steps || left == 0) {
       if (whole && ck == steps) {
@@ -500,20 +572,20 @@ int lut4_status(int reset) {
 }
 }  // namespace vq
 
-extern "C" {
-
 // How a product is cut: 8 * NT activation rows, weight tiles of 8 * RG rows, K slices, CTAs per slice.
 struct Lut4Plan {
   int nt, rg, tiles, steps, slices, ctas, max_parts, lda_s;
 };
-static Lut4Plan lut4_plan(int64_t M, int64_t N, int64_t K) {
+static Lut4Plan lut4_plan(int64_t M, int64_t N, int64_t K, bool wide) {
+  const int step = wide ? L4Step<true>::value : L4Step<false>::value;
   Lut4Plan q{};
   q.nt = (int)((M + 7) / 8);
   q.rg = q.nt <= 2 ? 4 : 2;                                  // partial tiles of both sets beside the activations
   q.tiles = (int)((N + 8 * q.rg - 1) / (8 * q.rg));
-  q.steps = (int)(K / L4_STEP);
-  static const int longest[5] = {0, 16, 8, 10, 8};           // steps of activations that fit behind table and ring
-  const int least_slices = (q.steps + longest[q.nt] - 1) / longest[q.nt];
+  q.steps = (int)(K / step);
+  // elements of an activation row that fit behind table and ring
+  static const int longest[2][5] = {{0, 2048, 1024, 1280, 1024}, {0, 2048, 1024, 1280, 896}};
+  const int fits = longest[wide][q.nt] / step, least_slices = (q.steps + fits - 1) / fits;
   // as few slices as that allows, or up to a quarter more where they use more of the SMs
   q.slices = least_slices;
   for (int n = least_slices + 1; n <= least_slices + least_slices / 4 && n <= kSmCount; ++n)
@@ -524,7 +596,8 @@ static Lut4Plan lut4_plan(int64_t M, int64_t N, int64_t K) {
   if (ctas > most) ctas = most;
   q.ctas = ctas < 1 ? 1 : (int)ctas;
   const int slice_max = (q.steps + q.slices - 1) / q.slices;
-  q.lda_s = slice_max * L4_STEP + L4_APAD;
+  // the rows' pitch spreads the lanes of a load over the banks: 32 bytes apart (packed, 8 bytes a lane), 64 (wide, 16)
+  q.lda_s = wide ? slice_max * step + (slice_max % 2 ? 64 : 32) : slice_max * step + L4_APAD;
   // a CTA has at least floor(total / ctas) consecutive steps of a slice, and a slice at most slice_max of a tile
   const int64_t least = total / q.ctas < 1 ? 1 : total / q.ctas;
   const int64_t per_slice = (slice_max - 1) / least + 2;
@@ -532,13 +605,92 @@ static Lut4Plan lut4_plan(int64_t M, int64_t N, int64_t K) {
   return q;
 }
 
+// The cut, tensor maps and launch of a product whose operands stand in `p`.
+template <bool WIDE>
+static int launch_row_stream(Lut4Params p, cudaStream_t st) {
+  const int64_t M = p.M, N = p.N, K = p.K;
+  const Lut4Plan q = lut4_plan(M, N, K, WIDE);
+  p.tiles = q.tiles; p.steps = q.steps; p.slices = q.slices; p.ctas = q.ctas; p.max_parts = q.max_parts; p.lda_s = q.lda_s;
+  while ((1 << p.bs_shift) < p.bs) ++p.bs_shift;
+  VQ_REQUIRE(p.slices <= 65535 && (int64_t)q.tiles * q.steps < (1ll << 31), "row stream: weight too large");
+  const int64_t most_ctas = q.ctas > L4_WARPS ? q.ctas : L4_WARPS;
+  p.small = ((int64_t)q.tiles * q.steps + 1) * most_ctas < (1ll << 32);
+  // Shared memory: the table must sit at shared address L4_TABLE_ADDR.  Dynamic memory starts somewhere in
+  // [1 KB, 4 KB) of the window (system + static variables), so reserving up to the table's end measured from
+  // 1 KB always suffices; scale slots and partial tiles (16 + 32 KB at most) fit before the table.
+  const int tile = q.rg * 8;
+  const int a_bytes = q.nt * 8 * q.lda_s * (int)sizeof(__nv_bfloat16);
+  const size_t smem = (size_t)L4_TABLE_ADDR + L4_TABLE_BYTES - 1024 + a_bytes + L4_WARPS * 2 * tile * 64;
+  constexpr int kMostSmem = (int)L4_TABLE_ADDR + L4_TABLE_BYTES - 1024 + 100352;   // 16 rows of 1088 elements + 64 KB
+  VQ_REQUIRE((int)smem <= kMostSmem, "row stream: internal error: %d bytes of shared memory", (int)smem);
+  CUtensorMap map_w, map_s;
+  if (int e = lut4_map(&map_w, p.w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, WIDE ? K * 2 : K / 2, N, 64, tile)) return e;
+  memset(&map_s, 0, sizeof(map_s));
+  p.tma_scales = (K / p.bs) % 8 == 0 && (reinterpret_cast<uintptr_t>(p.w_scale) & 15) == 0;
+  if (p.tma_scales)
+    if (int e = lut4_map(&map_s, p.w_scale, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, K / p.bs, N, 8, tile)) return e;
+  static unsigned long long configured = 0;
+  if (first_call_on_device(&configured)) {
+    cudaFuncSetAttribute(gemm_lut4_kernel<WIDE, 1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
+    cudaFuncSetAttribute(gemm_lut4_kernel<WIDE, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
+    cudaFuncSetAttribute(gemm_lut4_kernel<WIDE, 3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
+    cudaFuncSetAttribute(gemm_lut4_kernel<WIDE, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
+  }
+  const dim3 grid((unsigned)q.ctas, (unsigned)q.slices);
+  if (q.nt == 1) gemm_lut4_kernel<WIDE, 1, 4><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
+  else if (q.nt == 2) gemm_lut4_kernel<WIDE, 2, 4><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
+  else if (q.nt == 3) gemm_lut4_kernel<WIDE, 3, 2><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
+  else gemm_lut4_kernel<WIDE, 4, 2><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
+  return check_launch("gemm_lut4_kernel");
+}
+
+extern "C" {
+
 int64_t vq_gemm_lut4_workspace_floats(int64_t M, int64_t N, int64_t K) {
-  if (M <= 0 || N <= 0 || K <= 0 || M > 32 || K % L4_STEP) return 0;
-  const Lut4Plan q = lut4_plan(M, N, K);
+  if (M <= 0 || N <= 0 || K <= 0 || M > 32 || K % 128) return 0;
+  const Lut4Plan q = lut4_plan(M, N, K, false);
   return (int64_t)q.tiles * q.max_parts * (q.nt * 8) * (q.rg * 8);
 }
 
 int64_t vq_gemm_lut4_counters(int64_t N) { return N <= 0 ? 0 : (N + 15) / 16; }
+
+int64_t vq_gemm_mx_rows_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  if (M <= 0 || N <= 0 || K <= 0 || M > 32 || K % 32) return 0;
+  const Lut4Plan q = lut4_plan(M, N, K, true);
+  return ((int64_t)q.tiles * q.max_parts * (q.nt * 8) * (q.rg * 8) + q.tiles) * 4;
+}
+
+int vq_gemm_mx_rows(const void* a, const void* a_scale, const void* a_levels, int n_a_levels, const void* w,
+                    const void* w_scale, const void* w_levels, int64_t block_size, void* out, int out_dtype, int64_t M,
+                    int64_t N, int64_t K, const void* alpha, int alpha_dtype, const void* bias, int bias_dtype,
+                    void* workspace, void* stream) {
+  VQ_REQUIRE(M >= 0 && N >= 0 && K >= 0, "vq_gemm_mx_rows: negative extent");
+  if (M == 0 || N == 0) return VQ_OK;
+  VQ_REQUIRE(M <= 32 && K > 0 && K % 32 == 0, "vq_gemm_mx_rows: at most 32 activation rows, K a positive multiple of 32");
+  VQ_REQUIRE(block_size >= 8 && block_size < (1 << 30) && (block_size & (block_size - 1)) == 0 && K % block_size == 0,
+             "vq_gemm_mx_rows: the block size must be a power of two, at least 8, that divides K");
+  VQ_REQUIRE(a && a_scale && w && w_scale && out && workspace, "vq_gemm_mx_rows: null argument");
+  VQ_REQUIRE(((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(workspace)) & 15) == 0,
+             "vq_gemm_mx_rows: operands must be 16-byte aligned");
+  VQ_REQUIRE(a_levels == nullptr || (n_a_levels > 0 && n_a_levels <= 256),
+             "vq_gemm_mx_rows: an activation codebook has 1 to 256 entries");
+  VQ_REQUIRE(out_dtype >= VQ_BF16 && out_dtype <= VQ_F32, "vq_gemm_mx_rows: bad output dtype");
+  VQ_REQUIRE(N < (1ll << 31) && K < (1ll << 30), "vq_gemm_mx_rows: extent too large");
+  Lut4Params p{};
+  p.a = a; p.a_scale = a_scale; p.a_levels = a_levels; p.n_a_levels = n_a_levels;
+  p.w = static_cast<const uint8_t*>(w); p.w_scale = w_scale; p.w_levels = w_levels;
+  p.out = out; p.out_dt = out_dtype;
+  p.M = (int)M; p.N = (int)N; p.K = (int)K; p.bs = (int)block_size; p.lda = K;
+  p.alpha = alpha; p.alpha_dt = alpha_dtype; p.bias = bias; p.bias_dt = bias_dtype;
+  const Lut4Plan q = lut4_plan(M, N, K, true);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  p.counters = static_cast<int*>(workspace);
+  p.workspace = reinterpret_cast<float*>(p.counters + q.tiles);
+  // the tiles' counters belong to this call: products of several streams may run at the same time
+  if (cudaMemsetAsync(p.counters, 0, (size_t)q.tiles * sizeof(int), st) != cudaSuccess)
+    return fail(VQ_ECUDA, "vq_gemm_mx_rows: memset");
+  return launch_row_stream<true>(p, st);
+}
 
 int vq_pack_lut4(const void* codes, void* packed, int64_t rows, int64_t K, int* bad, void* stream) {
   VQ_REQUIRE(rows >= 0 && K >= 0 && K % 2 == 0, "vq_pack_lut4: K must be even");
@@ -575,40 +727,7 @@ int vq_gemm_lut4(const void* a, int64_t lda, const void* a_scale, const void* a_
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.bs = block_size; p.lda = lda;
   p.alpha = alpha; p.alpha_dt = alpha_dtype; p.bias = bias; p.bias_dt = bias_dtype;
   p.workspace = workspace; p.counters = counters;
-  const Lut4Plan q = lut4_plan(M, N, K);
-  p.tiles = q.tiles; p.steps = q.steps; p.slices = q.slices; p.ctas = q.ctas; p.max_parts = q.max_parts; p.lda_s = q.lda_s;
-  while ((1 << p.bs_shift) < block_size) ++p.bs_shift;
-  VQ_REQUIRE(p.slices <= 65535 && (int64_t)q.tiles * q.steps < (1ll << 31), "vq_gemm_lut4: weight too large");
-  const int64_t most_ctas = q.ctas > L4_WARPS ? q.ctas : L4_WARPS;
-  p.small = ((int64_t)q.tiles * q.steps + 1) * most_ctas < (1ll << 32);
-  // Shared memory: the table must sit at shared address L4_TABLE_ADDR.  Dynamic memory starts somewhere in
-  // [1 KB, 4 KB) of the window (system + static variables), so reserving up to the table's end measured from
-  // 1 KB always suffices; scale slots and partial tiles (16 + 32 KB at most) fit before the table.
-  const int tile = q.rg * 8;
-  const int a_bytes = q.nt * 8 * q.lda_s * (int)sizeof(__nv_bfloat16);
-  const size_t smem = (size_t)L4_TABLE_ADDR + L4_TABLE_BYTES - 1024 + a_bytes + L4_WARPS * 2 * tile * 64;
-  constexpr int kMostSmem = (int)L4_TABLE_ADDR + L4_TABLE_BYTES - 1024 + 99328;   // 32 rows of 1040 elements + 32 KB
-  VQ_REQUIRE((int)smem <= kMostSmem, "vq_gemm_lut4: internal error: %d bytes of shared memory", (int)smem);
-  CUtensorMap map_w, map_s;
-  if (int e = lut4_map(&map_w, w_packed, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 2, N, 64, tile)) return e;
-  memset(&map_s, 0, sizeof(map_s));
-  p.tma_scales = (K / block_size) % 8 == 0 && (reinterpret_cast<uintptr_t>(w_scale) & 15) == 0;
-  if (p.tma_scales)
-    if (int e = lut4_map(&map_s, w_scale, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, K / block_size, N, 8, tile)) return e;
-  static unsigned long long configured = 0;
-  if (first_call_on_device(&configured)) {
-    cudaFuncSetAttribute(gemm_lut4_kernel<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
-    cudaFuncSetAttribute(gemm_lut4_kernel<2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
-    cudaFuncSetAttribute(gemm_lut4_kernel<3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
-    cudaFuncSetAttribute(gemm_lut4_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
-  }
-  const dim3 grid((unsigned)q.ctas, (unsigned)q.slices);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (q.nt == 1) gemm_lut4_kernel<1, 4><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
-  else if (q.nt == 2) gemm_lut4_kernel<2, 4><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
-  else if (q.nt == 3) gemm_lut4_kernel<3, 2><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
-  else gemm_lut4_kernel<4, 2><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
-  return check_launch("gemm_lut4_kernel");
+  return launch_row_stream<false>(p, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"
