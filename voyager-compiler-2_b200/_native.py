@@ -238,6 +238,13 @@ def _cuda_device_of(values, found):
     return found
 
 
+def _current_device():
+    """The function that gives the calling thread's device ordinal."""
+    import torch
+
+    return getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+
+
 def device_guarded(fn):
     """Run ``fn`` with the device of its CUDA tensor arguments current, so that kernels launch on
     that device's current stream whatever device the caller had selected (a model whose layers are
@@ -247,13 +254,28 @@ def device_guarded(fn):
 
     import torch
 
+    tensor, current_device = torch.Tensor, _current_device()
+
+    # Every kernel call goes through here: device ordinals are compared as integers (a device object per operand and
+    # torch.cuda's checked accessors took 8 us of a call).
     @functools.wraps(fn)
     def call(*args, **kwargs):
-        device = _cuda_device_of(args, None)
-        device = _cuda_device_of(kwargs.values(), device)
-        if device is None or device.index == torch.cuda.current_device():
+        index = -1
+        for v in ((*args, *kwargs.values()) if kwargs else args):
+            if isinstance(v, tensor):
+                i = v.get_device() if v.is_cuda else -1
+            elif isinstance(v, (list, tuple)):
+                found = _cuda_device_of(v, None)
+                i = -1 if found is None else found.index
+            else:
+                continue
+            if i >= 0 and i != index:
+                if index >= 0:
+                    raise ValueError(f"operands live on different devices: cuda:{index} and cuda:{i}")
+                index = i
+        if index < 0 or index == current_device():
             return fn(*args, **kwargs)
-        with torch.cuda.device(device):
+        with torch.cuda.device(index):
             return fn(*args, **kwargs)
 
     return call

@@ -422,12 +422,12 @@ def quantize_fp8_transpose(input: torch.Tensor, scale: torch.Tensor, dtype="fp8_
     rows, cols = x.shape
     codes = torch.empty((rows, cols), dtype=torch.uint8, device=x.device)
     transpose = torch.empty((cols, rows), dtype=torch.uint8, device=x.device)
-    amax = torch.zeros((), dtype=torch.int32, device=x.device)
+    amax = torch.zeros(2, dtype=torch.bfloat16, device=x.device)   # one 32-bit word; the maximum ends in its low half
     N.check(N.lib().vq_transpose_quantize_fp8(x.data_ptr(), transpose.data_ptr(), codes.data_ptr(), amax.data_ptr(),
                                               _FORMATS[dtype], rows, 1, cols, cols, scale.data_ptr(),
                                               _dtype_id(scale.dtype), _stream()),
             "vq_transpose_quantize_fp8")
-    return _typed(codes, dtype), _typed(transpose, dtype), amax.to(torch.int16).view(torch.bfloat16)
+    return _typed(codes, dtype), _typed(transpose, dtype), amax[0]
 
 
 # ---------------------------------------------------------------------------

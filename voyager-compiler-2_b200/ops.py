@@ -11,6 +11,7 @@ Do not import this module in a process that has imported the reference's
 ``voyager_compiler.ops``: both define the ``quantized_ops`` namespace.
 """
 
+import functools
 import math
 from typing import List, Optional, Sequence, Tuple
 
@@ -38,8 +39,15 @@ def _dtype_id(dtype):
         raise TypeError(f"quantized_ops kernels take bfloat16, float16 or float32 tensors, not {dtype}") from None
 
 
+_current_device = N._current_device()
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle (without building a torch.cuda.Stream for it)."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def _ptr(t):
@@ -299,8 +307,12 @@ def _(input, scale, zero_point=None, axes=None, block_size=None, input_qmap=None
 # ---------------------------------------------------------------------------
 def _block_geometry(shape, axes, block_size):
     """``(VqBlocks, scale_shape)`` for blocks of ``block_size`` along one or two axes."""
+    return _block_geometry_of(tuple(shape), (axes,) if isinstance(axes, int) else tuple(axes), block_size)
+
+
+@functools.lru_cache(maxsize=256)
+def _block_geometry_of(shape, axes, block_size):
     nd = len(shape)
-    axes = [axes] if isinstance(axes, int) else list(axes)
     axes = sorted({a + nd if a < 0 else a for a in axes})
     if not axes or len(axes) > 2 or any(a < 0 or a >= nd for a in axes):
         raise NotImplementedError(f"blocks along axes {axes} of a {nd}-d tensor")
@@ -318,7 +330,7 @@ def _block_geometry(shape, axes, block_size):
     scale_shape = list(shape)
     for a in axes:
         scale_shape[a] = -(-shape[a] // block_size)
-    return b, scale_shape
+    return b, tuple(scale_shape)
 
 
 def _scale_rule(x, quant_max, power_of_two, scale_qmap, global_scale):
@@ -570,6 +582,7 @@ _ACT_LAYOUTS, _WGT_LAYOUTS, _OUT_LAYOUTS = ("xc", "cx"), ("kc", "ck"), ("xk", "k
 _IN_KIND = {torch.bfloat16: N.IN_BF16, torch.float16: N.IN_F16}
 
 
+@functools.lru_cache(maxsize=64)
 def _parse_layout(layout: str):
     operands, out = layout.split("->")
     act, wgt = operands.split(",")
@@ -615,7 +628,6 @@ def gemm_tn(a: torch.Tensor, b: torch.Tensor, *, out_dtype=None, alpha=None, bia
         a = torch.nn.functional.pad(a, (0, pad))
         b = torch.nn.functional.pad(b, (0, pad))
         k += pad
-    batch_shape = torch.broadcast_shapes(a.shape[:-2], b.shape[:-2])
     if b.dim() == 2:
         # shared weight: fold the batch into the rows
         a2 = a.reshape(-1, k).contiguous()
@@ -623,6 +635,7 @@ def gemm_tn(a: torch.Tensor, b: torch.Tensor, *, out_dtype=None, alpha=None, bia
         batch, rows = 1, a2.shape[0]
         stride_a = stride_b = 0
     else:
+        batch_shape = torch.broadcast_shapes(a.shape[:-2], b.shape[:-2])
         a2 = a.expand(*batch_shape, m, k).reshape(-1, m, k).contiguous()
         b2 = b.expand(*batch_shape, n, k).reshape(-1, n, k).contiguous()
         batch, rows = a2.shape[0], m
