@@ -213,6 +213,12 @@ int vq_amax_history_update(void* ring, int dtype, int64_t length, int64_t channe
 int vq_hadamard_rotate(const void* in, void* out, int dtype, const float* matrix, int64_t O, int64_t A,
                        int64_t I, void* stream);
 
+/* hessian_inverse_chol's factorisation (quantization/gptq.py:37-75) in one elimination: W holds the damped Hessian with rows
+ * and columns in reverse order, [n, n] float32, n a multiple of 128 (pad with an identity block at the end); on return its
+ * lower triangle is L^-1 where W = L L^T, whose reverse in rows and columns is the upper Cholesky factor of the
+ * Hessian's inverse.  panel: n * 128 floats of workspace; *info (device) becomes 1 if a pivot was not positive. */
+int vq_gptq_factor(float* W, float* panel, int64_t n, int* info, void* stream);
+
 /* One block of the GPTQ column sweep -- quantization/gptq.py: block_scale (85-143)
  * and quantize_block (189-220), as compensate_weight (223-308) calls them.
  * work/out are fp32 [rows, K]; columns [start, start+n) (n <= 128) are rounded one

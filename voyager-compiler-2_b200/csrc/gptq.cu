@@ -8,11 +8,13 @@
 //      error over its pivot U[c][c] is propagated into the block's later
 //      columns with U's row c (U = upper Cholesky factor of the inverse Hessian);
 //   3. the trailing columns receive  work[:, end:] -= deltas @ U[start:end, end:].
-// Rows never interact, so one thread owns one row: its slice of the block lives
-// in registers, U's diagonal tile is broadcast from shared memory, and every
-// arithmetic step is a separately rounded fp32 operation in the order the
-// reference's column loop performs them.
+// Rows never interact.  Eight lanes share a row, each with four neighbouring columns of every 32 in registers; U's
+// diagonal tile stands in shared memory, and every arithmetic step is a separately rounded fp32 operation in
+// the order the reference's column loop performs them.  The columns are a serial chain -- quotient, rounding,
+// difference, quotient by the pivot, broadcast, update -- and that latency is what the kernel's time is: 128 columns
+// of 4096 rows take BLOCKNOW us, 387 us with a thread per row and its 128 values updated one by one.
 
+#include "gptq_tile.cuh"
 #include "quantize_shared.cuh"
 
 namespace vq {
@@ -20,7 +22,8 @@ namespace {
 
 constexpr float kEps = 1e-12f;  // the reference's EPS clamp on scales and pivots
 constexpr int kMaxBlock = 128;
-constexpr int kRowsPerCta = 32;   // one warp per CTA: twice the CTAs of a 64-row split, and up to 3 CTAs share an SM at 64 KB of shared memory each
+constexpr int kBlockThreads = 128;
+constexpr int kRowsPerCta = kBlockThreads / 8;
 constexpr int kShrinkCandidates = 5;
 
 struct GptqBlockParams {
@@ -34,57 +37,80 @@ struct GptqBlockParams {
   int affine;           // 0: microscaling scale; 1: group-wise affine (scale + zero point)
   float quant_min, quant_max;
   int shrink;
+  int vec;              // rows of work, out and deltas are whole 16-byte pieces
   Round scale_round;    // rounding of the scale (microscaling)
   Round round;          // element grid
 };
 
+template <int MODE>
 __device__ __forceinline__ float grid_value(const Round& r, float w, float scale, float zero, bool affine) {
   // quantize(w / scale [+ zero]) then back to the weight's units
   float y = __fdiv_rn(w, scale);
   if (affine) y = __fadd_rn(y, zero);
-  float code = apply_round(r, y, 0);
+  float code = apply_round<MODE>(r, y, 0);
   if (affine) code = __fsub_rn(code, zero);
   return __fmul_rn(code, scale);
 }
 
-template <int MAXN>
-__global__ void __launch_bounds__(kRowsPerCta)
-gptq_block_kernel(GptqBlockParams p) {
-  extern __shared__ float tile[];  // U[start:start+n, start:start+n], row-major n x n
+// NQ: groups of 32 columns.  MODE: the element grid's rounding at compile time, or -1.
+template <int NQ, int MODE>
+__global__ void __launch_bounds__(kBlockThreads)
+gptq_block_kernel(const __grid_constant__ GptqBlockParams p) {
+  constexpr int W = 32 * NQ;
+  extern __shared__ __align__(16) float tile[];  // strictly upper part of U[start:start+n, start:start+n], W x W
   __shared__ uint16_t s_steps[2][2 * VQ_MAX_STEPS];
-  stage_steps(p.round, s_steps[0]);
-  stage_steps(p.scale_round, s_steps[1]);
+  __shared__ float s_pivot[W];
+  Round round = p.round, scale_round = p.scale_round;
+  stage_steps(round, s_steps[0]);
+  stage_steps(scale_round, s_steps[1]);
   const int n = p.n;
-  for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-    const int r = t / n, c = t - r * n;
-    tile[t] = p.U[(int64_t)(p.start + r) * p.K + p.start + c];
+  for (int t = threadIdx.x; t < W * W; t += kBlockThreads) {
+    const int r = t / W, c = t - r * W;
+    tile[t] = r < c && c < n ? p.U[(int64_t)(p.start + r) * p.K + p.start + c] : 0.0f;
   }
+  for (int t = threadIdx.x; t < W; t += kBlockThreads)
+    s_pivot[t] = t < n ? fmaxf(p.U[(int64_t)(p.start + t) * p.K + p.start + t], kEps) : 1.0f;
   __syncthreads();
-  const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= p.rows) return;
+  const int lane = threadIdx.x & 31, l = lane & 7, first = lane & 24;
+  const int64_t row = (int64_t)blockIdx.x * kRowsPerCta + (threadIdx.x >> 3);
+  const bool live = row < p.rows;
 
-  float w[MAXN];
-  float* wrow = p.work + row * p.K + p.start;
+  float w[4 * NQ];   // column 32 q + 4 l + e
+  const float* wrow = p.work + (live ? row : p.rows - 1) * p.K + p.start;
 #pragma unroll
-  for (int c = 0; c < MAXN; ++c) w[c] = c < n ? wrow[c] : 0.0f;
+  for (int q = 0; q < NQ; ++q) {
+    const int c = 32 * q + 4 * l;
+    if (p.vec) {
+      const float4 v = c < n ? *reinterpret_cast<const float4*>(wrow + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[4 * q + e] = c + e < n ? wrow[c + e] : 0.0f;
+    }
+  }
 
   // ---- per-row scale (and zero point) from the block as compensated so far ----
+  const bool affine = p.affine != 0;
   float scale, zero = 0.0f;
-  if (p.affine) {
-    float lo = w[0], hi = w[0];
+  if (affine) {
+    float lo = __uint_as_float(0x7FC00000u), hi = lo;   // a NaN is no minimum or maximum
 #pragma unroll
-    for (int c = 1; c < MAXN; ++c)
-      if (c < n) { lo = fminf(lo, w[c]); hi = fmaxf(hi, w[c]); }
+    for (int i = 0; i < 4 * NQ; ++i)
+      if (32 * (i >> 2) + 4 * l + (i & 3) < n) { lo = fminf(lo, w[i]); hi = fmaxf(hi, w[i]); }
+    for (int off = 1; off < 8; off <<= 1) {
+      lo = fminf(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, off));
+      hi = fmaxf(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, off));
+    }
     scale = __fdiv_rn(__fsub_rn(hi, lo), __fsub_rn(p.quant_max, p.quant_min));
     scale = scale > 0.0f ? scale : 1.0f;
     zero = __fadd_rn(__fdiv_rn(-lo, scale), p.quant_min);
   } else {
     uint32_t m = 0;
 #pragma unroll
-    for (int c = 0; c < MAXN; ++c)
-      if (c < n) m = max(m, abs_bits(w[c]));
+    for (int i = 0; i < 4 * NQ; ++i) m = max(m, abs_bits(w[i]));   // columns past the block are zeros
+    for (int off = 1; off < 8; off <<= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, off));
     float base = __fdiv_rn(__uint_as_float(m), p.quant_max);
-    if (p.scale_round.mode != VQ_ROUND_NONE) base = apply_round(p.scale_round, base, 0);
+    if (scale_round.mode != VQ_ROUND_NONE) base = apply_round(scale_round, base, 0);
     base = base > 0.0f ? base : 1.0f;
     base = fmaxf(base, kEps);
     scale = base;
@@ -96,37 +122,91 @@ gptq_block_kernel(GptqBlockParams p) {
         float s = base;
         if (f > 0) {
           s = __bfloat162float(__float2bfloat16_rn(__fmul_rn(base, factors[f])));
-          s = apply_round(p.scale_round, s, 0);
+          s = apply_round(scale_round, s, 0);
           s = fmaxf(s, kEps);
         }
-        float err = 0.0f;
+        float err = 0.0f;   // the columns' terms in ascending order
 #pragma unroll
-        for (int c = 0; c < MAXN; ++c)
-          if (c < n) {
-            const float d = __fsub_rn(w[c], grid_value(p.round, w[c], s, 0.0f, false));
-            err = __fadd_rn(err, __fmul_rn(__fmul_rn(d, d), p.salience[p.start + c]));
+        for (int q = 0; q < NQ; ++q) {
+          float term[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int c = 32 * q + 4 * l + e;
+            const float d = __fsub_rn(w[4 * q + e], grid_value<MODE>(round, w[4 * q + e], s, 0.0f, false));
+            term[e] = c < n ? __fmul_rn(__fmul_rn(d, d), p.salience[p.start + c]) : 0.0f;
           }
+          for (int ll = 0; ll < 8; ++ll)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float t = __shfl_sync(0xFFFFFFFFu, term[e], first + ll);
+              if (32 * q + 4 * ll + e < n) err = __fadd_rn(err, t);
+            }
+        }
         if (f == 0 || err < best_err) { best_err = err; scale = s; }
       }
     }
   }
 
   // ---- column sweep ----
+  float level[4 * NQ], step[4 * NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+#pragma unroll 1
+    for (int ll = 0; ll < 8; ++ll) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int c = 32 * q + 4 * ll + e;   // lane ll of the row has it
+        const float g = grid_value<MODE>(round, w[4 * q + e], scale, zero, affine);
+        const float mine = __fdiv_rn(__fsub_rn(w[4 * q + e], g), s_pivot[c]);
+        const float delta = __shfl_sync(0xFFFFFFFFu, mine, first + ll);
+        if (l == ll) { level[4 * q + e] = g; step[4 * q + e] = mine; }
+        const float* u = tile + c * W + 4 * l;
+#pragma unroll
+        for (int q2 = q; q2 < NQ; ++q2) {   // zeros up to column c itself
+          const float4 v = *reinterpret_cast<const float4*>(u + 32 * q2);
+          w[4 * q2] = __fsub_rn(w[4 * q2], __fmul_rn(delta, v.x));
+          w[4 * q2 + 1] = __fsub_rn(w[4 * q2 + 1], __fmul_rn(delta, v.y));
+          w[4 * q2 + 2] = __fsub_rn(w[4 * q2 + 2], __fmul_rn(delta, v.z));
+          w[4 * q2 + 3] = __fsub_rn(w[4 * q2 + 3], __fmul_rn(delta, v.w));
+        }
+      }
+    }
+  }
+  if (!live) return;
   float* orow = p.out + row * p.K + p.start;
   float* drow = p.deltas + row * n;
 #pragma unroll
-  for (int c = 0; c < MAXN; ++c) {
-    if (c < n) {
-      const float level = grid_value(p.round, w[c], scale, zero, p.affine != 0);
-      const float pivot = fmaxf(tile[c * n + c], kEps);
-      const float delta = __fdiv_rn(__fsub_rn(w[c], level), pivot);
-      orow[c] = level;
-      drow[c] = delta;
+  for (int q = 0; q < NQ; ++q) {
+    const int c = 32 * q + 4 * l;
+    if (p.vec) {
+      if (c < n) {
+        *reinterpret_cast<float4*>(orow + c) = make_float4(level[4 * q], level[4 * q + 1], level[4 * q + 2], level[4 * q + 3]);
+        *reinterpret_cast<float4*>(drow + c) = make_float4(step[4 * q], step[4 * q + 1], step[4 * q + 2], step[4 * q + 3]);
+      }
+    } else {
 #pragma unroll
-      for (int j = c + 1; j < MAXN; ++j)
-        if (j < n) w[j] = __fsub_rn(w[j], __fmul_rn(delta, tile[c * n + j]));
+      for (int e = 0; e < 4; ++e)
+        if (c + e < n) { orow[c + e] = level[4 * q + e]; drow[c + e] = step[4 * q + e]; }
     }
   }
+}
+
+// The same update on whole 16-byte pieces: 128 x 128 tiles, the sums in the same order.  4096 rows, 128 columns of errors
+// and 3968 trailing ones: UPDBIG us, 180 us as 64 x 64 tiles (23 TFLOP/s).
+__global__ void __launch_bounds__(256, 2)
+gptq_update_tiles_kernel(float* __restrict__ work, const float* __restrict__ deltas, const float* __restrict__ U,
+                         int64_t rows, int64_t K, int start, int n, int end) {
+  __shared__ __align__(16) GtSmem s;
+  const int64_t r0 = (int64_t)blockIdx.y * kGt, j0 = (int64_t)end + (int64_t)blockIdx.x * kGt;
+  const int live_rows = (int)min((int64_t)kGt, rows - r0), live_cols = (int)min((int64_t)kGt, K - j0);
+  uint64_t acc[8][4];
+  gt_multiply<false>(acc, s, deltas + r0 * n, n, U + (int64_t)start * K + j0, K, live_rows, live_cols, n);
+  gt_each(acc, [&](int r, int c, float4 v) {
+    if (r >= live_rows || c >= live_cols) return;
+    float4* dst = reinterpret_cast<float4*>(work + (r0 + r) * K + j0 + c);
+    const float4 old = *dst;
+    *dst = make_float4(__fsub_rn(old.x, v.x), __fsub_rn(old.y, v.y), __fsub_rn(old.z, v.z), __fsub_rn(old.w, v.w));
+  });
 }
 
 // work[r][end + j] -= sum_c deltas[r][c] * U[start + c][end + j], c ascending, fp32.
@@ -208,13 +288,22 @@ extern "C" int vq_gptq_block(float* work, float* out, float* deltas, const float
   p.round = make_round(round);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int grid = (int)((rows + kRowsPerCta - 1) / kRowsPerCta);
-  const size_t smem = (size_t)n * n * sizeof(float);
+  p.vec = K % 4 == 0 && start % 4 == 0 && n % 4 == 0 &&
+          ((reinterpret_cast<uintptr_t>(work) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(deltas)) & 15) == 0;
   static unsigned long long configured = 0;
-  if (first_call_on_device(&configured))
-    cudaFuncSetAttribute(gptq_block_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 128 * 4);
-  if (n <= 32) gptq_block_kernel<32><<<grid, kRowsPerCta, smem, st>>>(p);
-  else if (n <= 64) gptq_block_kernel<64><<<grid, kRowsPerCta, smem, st>>>(p);
-  else gptq_block_kernel<128><<<grid, kRowsPerCta, smem, st>>>(p);
+  if (first_call_on_device(&configured)) {
+    cudaFuncSetAttribute(gptq_block_kernel<4, VQ_ROUND_INT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 128 * 4);
+    cudaFuncSetAttribute(gptq_block_kernel<4, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 128 * 4);
+  }
+  const int width = n <= 32 ? 32 : n <= 64 ? 64 : 128;
+  const size_t smem = (size_t)width * width * sizeof(float);
+#define VQ_BLOCK(NQ)                                                                                    \
+  (p.round.mode == VQ_ROUND_INT ? gptq_block_kernel<NQ, VQ_ROUND_INT><<<grid, kBlockThreads, smem, st>>>(p) \
+                                : gptq_block_kernel<NQ, -1><<<grid, kBlockThreads, smem, st>>>(p))
+  if (width == 32) VQ_BLOCK(1);
+  else if (width == 64) VQ_BLOCK(2);
+  else VQ_BLOCK(4);
+#undef VQ_BLOCK
   return check_launch("gptq_block_kernel");
 }
 
@@ -224,6 +313,13 @@ extern "C" int vq_gptq_update(float* work, const float* deltas, const float* U, 
   const int64_t end = start + n;
   if (rows == 0 || end == K) return VQ_OK;
   VQ_REQUIRE(work && deltas && U, "vq_gptq_update: null argument");
+  if (K % 4 == 0 && start % 4 == 0 && n % 4 == 0 && rows < (1ll << 22) &&
+      ((reinterpret_cast<uintptr_t>(work) | reinterpret_cast<uintptr_t>(deltas) | reinterpret_cast<uintptr_t>(U)) & 15) == 0) {
+    const dim3 tiles((unsigned)((K - end + kGt - 1) / kGt), (unsigned)((rows + kGt - 1) / kGt));
+    gptq_update_tiles_kernel<<<tiles, 256, 0, static_cast<cudaStream_t>(stream)>>>(work, deltas, U, rows, K, (int)start,
+                                                                                   (int)n, (int)end);
+    return check_launch("gptq_update_tiles_kernel");
+  }
   dim3 grid((unsigned)((K - end + kUpdTile - 1) / kUpdTile), (unsigned)((rows + kUpdTile - 1) / kUpdTile));
   gptq_update_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(work, deltas, U, rows, K, (int)start,
                                                                           (int)n, (int)end);

@@ -1,0 +1,147 @@
+// The factor a GPTQ sweep walks along: U upper triangular with U^T U = H^-1 (hessian_inverse_chol, reference
+// quantization/gptq.py:37-75), in one elimination.
+//
+// With J the exchange of rows and columns and J H J = L L^T, U = J L^-1 J: one Cholesky factorisation and one triangular
+// inverse, k^3 / 3 multiply-adds each, where factor - invert - factor again takes four times that.  Both
+// run here as one blocked Gauss-Jordan elimination in place on W = J H J (lower triangle): step j, for 128-row blocks,
+//   diag    W[j,j] = L_jj^-1                                         (one CTA)
+//   panel   P[i] = W[i,j] L_jj^-T for i > j;  W[j,k] = L_jj^-1 W[j,k] for k < j
+//   update  W[i,k] -= P[i] P[k]^T for j < k <= i;  W[i,j] = -P[i] L_jj^-1;  W[i,k] -= P[i] W[j,k] for k < j
+// and leaves L^-1 in W.  All of it is float32 FMAs: the update is bound by them, the diagonal blocks (one after the
+// other, 128 columns each) by latency.  K = 4096: FACTORNOW ms (diag DIAGNOW us, panel PANELNOW us, update UPDATENOW us a
+// step on average); factor, inverse and second factor from the library took 12 ms.
+#include "gptq_tile.cuh"
+
+namespace vq {
+namespace {
+
+// One 128 x 128 block: 512 threads own 4 x 8 elements each in registers.  Column c's raw values and row c's go through
+// shared memory (two buffers, one barrier per column); every thread then eliminates its own elements.
+__global__ void __launch_bounds__(512, 1)
+factor_diag_kernel(float* __restrict__ W, int64_t n, int j, int* __restrict__ info) {
+  __shared__ float col[2][128], row[2][128];
+  float* base = W + ((int64_t)j * 128) * n + (int64_t)j * 128;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float w[4][8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 x = *reinterpret_cast<const float4*>(base + (ty * 4 + i) * n + tx * 8);
+    const float4 y = *reinterpret_cast<const float4*>(base + (ty * 4 + i) * n + tx * 8 + 4);
+    w[i][0] = x.x; w[i][1] = x.y; w[i][2] = x.z; w[i][3] = x.w;
+    w[i][4] = y.x; w[i][5] = y.y; w[i][6] = y.z; w[i][7] = y.w;
+  }
+  bool bad = false;
+  for (int cb = 0; cb < 16; ++cb) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int c = cb * 8 + u;
+      float* pc = col[u & 1];
+      float* pr = row[u & 1];
+      if (tx == cb) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) pc[ty * 4 + i] = w[i][u];
+      }
+      if (ty == cb * 2 + (u >> 2)) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) pr[tx * 8 + k] = w[u & 3][k];
+      }
+      __syncthreads();
+      const float pivot = pc[c];
+      bad |= !(pivot > 0.0f);
+      const float inv = __frcp_rn(__fsqrt_rn(pivot));
+      float l[4], v[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) l[i] = __fmul_rn(pc[ty * 4 + i], inv);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int kk = tx * 8 + k;
+        // columns right of c: L's column (by symmetry); left of it: row c of the inverse; c itself: its diagonal
+        v[k] = kk == c ? inv : __fmul_rn(kk > c ? pc[kk] : pr[kk], inv);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int ii = ty * 4 + i;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int kk = tx * 8 + k;
+          const float old = kk == c ? 0.0f : w[i][k];
+          if (ii > c) w[i][k] = fmaf(-l[i], v[k], old);
+          else if (ii == c && kk <= c) w[i][k] = v[k];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (tx * 8 + k > ty * 4 + i) w[i][k] = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    *reinterpret_cast<float4*>(base + (ty * 4 + i) * n + tx * 8) = make_float4(w[i][0], w[i][1], w[i][2], w[i][3]);
+    *reinterpret_cast<float4*>(base + (ty * 4 + i) * n + tx * 8 + 4) = make_float4(w[i][4], w[i][5], w[i][6], w[i][7]);
+  }
+  if (bad && threadIdx.x == 0) atomicExch(info, 1);
+}
+
+// blockIdx.x < nb - j - 1: P[i] = W[i,j] L_jj^-T, i = j + 1 + blockIdx.x; the others: W[j,k] = L_jj^-1 W[j,k].
+__global__ void __launch_bounds__(256, 2)
+factor_panel_kernel(float* __restrict__ W, float* __restrict__ P, int64_t n, int j) {
+  __shared__ __align__(16) GtSmem s;
+  const int nb = (int)(n / 128), below = nb - j - 1;
+  const float* inv = W + ((int64_t)j * 128) * n + (int64_t)j * 128;
+  uint64_t acc[8][4];
+  if ((int)blockIdx.x < below) {
+    const int i = j + 1 + blockIdx.x;
+    gt_multiply<true>(acc, s, W + ((int64_t)i * 128) * n + (int64_t)j * 128, n, inv, n, 128, 128, 128);
+    float* out = P + (int64_t)i * 128 * 128;
+    gt_each(acc, [&](int r, int c, float4 v) { *reinterpret_cast<float4*>(out + r * 128 + c) = v; });
+  } else {
+    float* tile = W + ((int64_t)j * 128) * n + (int64_t)(blockIdx.x - below) * 128;
+    gt_multiply<false>(acc, s, inv, n, tile, n, 128, 128, 128);
+    __syncthreads();   // the tile has been read
+    gt_each(acc, [&](int r, int c, float4 v) { *reinterpret_cast<float4*>(tile + r * n + c) = v; });
+  }
+}
+
+// One tile (i, k), i > j, k <= i: blockIdx.x counts them row by row.
+__global__ void __launch_bounds__(256, 2)
+factor_update_kernel(float* __restrict__ W, const float* __restrict__ P, int64_t n, int j) {
+  __shared__ __align__(16) GtSmem s;
+  int i = j + 1, k = blockIdx.x;
+  while (k > i) { k -= i + 1; ++i; }
+  float* tile = W + ((int64_t)i * 128) * n + (int64_t)k * 128;
+  const float* p = P + (int64_t)i * 128 * 128;
+  uint64_t acc[8][4];
+  if (k > j) gt_multiply<true>(acc, s, p, 128, P + (int64_t)k * 128 * 128, 128, 128, 128, 128);
+  else gt_multiply<false>(acc, s, p, 128, W + ((int64_t)j * 128) * n + (int64_t)k * 128, n, 128, 128, 128);
+  const bool fresh = k == j;   // the panel's place: what stood here is in P
+  gt_each(acc, [&](int r, int c, float4 v) {
+    float4* dst = reinterpret_cast<float4*>(tile + r * n + c);
+    const float4 old = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : *dst;
+    *dst = make_float4(old.x - v.x, old.y - v.y, old.z - v.z, old.w - v.w);
+  });
+}
+
+}  // namespace
+}  // namespace vq
+
+using namespace vq;
+
+extern "C" int vq_gptq_factor(float* W, float* panel, int64_t n, int* info, void* stream) {
+  VQ_REQUIRE(n >= 0 && n % 128 == 0 && n <= (1 << 20), "vq_gptq_factor: the extent must be a multiple of 128");
+  if (n == 0) return VQ_OK;
+  VQ_REQUIRE(W && panel && info, "vq_gptq_factor: null argument");
+  VQ_REQUIRE(((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(panel)) & 15) == 0, "vq_gptq_factor: misaligned buffers");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (cudaMemsetAsync(info, 0, sizeof(int), st) != cudaSuccess) return fail(VQ_ECUDA, "vq_gptq_factor: memset");
+  const int nb = (int)(n / 128);
+  for (int j = 0; j < nb; ++j) {
+    factor_diag_kernel<<<1, 512, 0, st>>>(W, n, j, info);
+    if (nb > 1) factor_panel_kernel<<<nb - 1, 256, 0, st>>>(W, panel, n, j);
+    // tiles (i, 0 .. i) for i = j + 1 .. nb - 1
+    const int64_t tiles = (int64_t)nb * (nb + 1) / 2 - (int64_t)(j + 1) * (j + 2) / 2;
+    if (tiles > 0) factor_update_kernel<<<(unsigned)tiles, 256, 0, st>>>(W, panel, n, j);
+  }
+  return check_launch("gptq factor");
+}

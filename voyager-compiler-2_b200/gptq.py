@@ -4,8 +4,8 @@ Mirrors the single-weight step of the reference's ``quantization/gptq.py``:
 ``hessian_inverse_chol`` (``:37-75``), ``salience_order`` (``:146-186``) and
 ``compensate_weight`` (``:223-308``).  The Hessian ``X^T X`` is accumulated on the
 tensor cores (bf16 operands, fp32 accumulation, like the reference's CUDA
-``addmm``, ``:697-704``); the Cholesky factorisations are torch.linalg calls, as
-in the reference; the block scale, the column-by-column rounding with error
+``addmm``, ``:697-704``); the inverse's Cholesky factor comes from one blocked
+elimination (``csrc/gptq_factor.cu``); the block scale, the column-by-column rounding with error
 propagation and the trailing update are hand-written kernels (``csrc/gptq.cu``).
 
 ``compensate_weight_affine`` is the group-wise asymmetric variant (scale and
@@ -46,13 +46,32 @@ def hessian_inverse_chol(hessian, tokens, damping):
     for escalation in (1, 10, 100, 1000, 10000):
         h.diagonal().add_((escalation - applied) * damp)
         applied = escalation
-        lower, info = torch.linalg.cholesky_ex(h)
+        factor, info = _inverse_factor(h)
         if int(info) != 0:
             continue
         if escalation > 1:
             logger.warning("Hessian needed %dx the requested damping to invert: it is rank-deficient", escalation)
-        return torch.linalg.cholesky(torch.cholesky_inverse(lower), upper=True)
+        return factor() if callable(factor) else factor
     raise torch.linalg.LinAlgError("Hessian not positive-definite")
+
+
+@N.device_guarded
+def _inverse_factor(h):
+    """``(U, info)`` with ``U^T U = h^-1``, ``U`` upper triangular (or a function that computes it); ``info`` is not 0
+    if ``h`` is not positive definite."""
+    if not h.is_cuda or h.dtype != torch.float32 or h.dim() != 2 or h.shape[0] != h.shape[1] or h.shape[0] == 0:
+        lower, info = torch.linalg.cholesky_ex(h)
+        return (lambda: torch.linalg.cholesky(torch.cholesky_inverse(lower), upper=True)), info
+    # with rows and columns reversed, the inverse of h's lower factor is the upper factor of the inverse
+    k = h.shape[0]
+    n = -(-k // 128) * 128
+    work = torch.flip(h, (0, 1)) if n == k else torch.eye(n, dtype=h.dtype, device=h.device)
+    if n != k:
+        work[:k, :k] = torch.flip(h, (0, 1))
+    panel = torch.empty(n * 128, dtype=torch.float32, device=h.device)
+    info = torch.empty((), dtype=torch.int32, device=h.device)
+    N.check(N.lib().vq_gptq_factor(work.data_ptr(), panel.data_ptr(), n, info.data_ptr(), _stream()), "vq_gptq_factor")
+    return torch.flip(work.tril_()[:k, :k], (0, 1)), info
 
 
 def salience_order(hessian, columns, within_block, block_size):
@@ -81,7 +100,7 @@ def sweep(weight, hinv_chol, block_size, qmap, scale_qmap=None, quant_max=None, 
     work = weight.float().contiguous().clone()
     rows, K = work.shape
     U = hinv_chol.float().contiguous()
-    out = torch.zeros_like(work)
+    out = torch.empty_like(work)
     deltas = torch.empty(rows, min(block_size, K), dtype=torch.float32, device=work.device)
     spec = R.table_round(qmap)
     sspec = R.none_round() if scale_qmap is None else R.table_round(scale_qmap)
