@@ -12,7 +12,7 @@
 // diagonal tile stands in shared memory, and every arithmetic step is a separately rounded fp32 operation in
 // the order the reference's column loop performs them.  The columns are a serial chain -- quotient, rounding,
 // difference, quotient by the pivot, broadcast, update -- and that latency is what the kernel's time is: 128 columns
-// of 4096 rows take BLOCKNOW us, 387 us with a thread per row and its 128 values updated one by one.
+// of 4096 rows take 38 us, 387 us with a thread per row and its 128 values updated one by one.
 
 #include "gptq_tile.cuh"
 #include "quantize_shared.cuh"
@@ -156,18 +156,20 @@ gptq_block_kernel(const __grid_constant__ GptqBlockParams p) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int c = 32 * q + 4 * ll + e;   // lane ll of the row has it
+        float4 u[NQ];   // fetched before the quotients, which it does not depend on; zeros up to column c itself
+#pragma unroll
+        for (int q2 = q; q2 < NQ; ++q2) u[q2] = *reinterpret_cast<const float4*>(tile + c * W + 4 * l + 32 * q2);
+        const float pivot = s_pivot[c];
         const float g = grid_value<MODE>(round, w[4 * q + e], scale, zero, affine);
-        const float mine = __fdiv_rn(__fsub_rn(w[4 * q + e], g), s_pivot[c]);
+        const float mine = __fdiv_rn(__fsub_rn(w[4 * q + e], g), pivot);
         const float delta = __shfl_sync(0xFFFFFFFFu, mine, first + ll);
         if (l == ll) { level[4 * q + e] = g; step[4 * q + e] = mine; }
-        const float* u = tile + c * W + 4 * l;
 #pragma unroll
-        for (int q2 = q; q2 < NQ; ++q2) {   // zeros up to column c itself
-          const float4 v = *reinterpret_cast<const float4*>(u + 32 * q2);
-          w[4 * q2] = __fsub_rn(w[4 * q2], __fmul_rn(delta, v.x));
-          w[4 * q2 + 1] = __fsub_rn(w[4 * q2 + 1], __fmul_rn(delta, v.y));
-          w[4 * q2 + 2] = __fsub_rn(w[4 * q2 + 2], __fmul_rn(delta, v.z));
-          w[4 * q2 + 3] = __fsub_rn(w[4 * q2 + 3], __fmul_rn(delta, v.w));
+        for (int q2 = q; q2 < NQ; ++q2) {
+          w[4 * q2] = __fsub_rn(w[4 * q2], __fmul_rn(delta, u[q2].x));
+          w[4 * q2 + 1] = __fsub_rn(w[4 * q2 + 1], __fmul_rn(delta, u[q2].y));
+          w[4 * q2 + 2] = __fsub_rn(w[4 * q2 + 2], __fmul_rn(delta, u[q2].z));
+          w[4 * q2 + 3] = __fsub_rn(w[4 * q2 + 3], __fmul_rn(delta, u[q2].w));
         }
       }
     }
@@ -191,8 +193,8 @@ gptq_block_kernel(const __grid_constant__ GptqBlockParams p) {
   }
 }
 
-// The same update on whole 16-byte pieces: 128 x 128 tiles, the sums in the same order.  4096 rows, 128 columns of errors
-// and 3968 trailing ones: UPDBIG us, 180 us as 64 x 64 tiles (23 TFLOP/s).
+// The same update on whole 16-byte pieces: 128 x 128 tiles, the sums in the same order.  Averaged over
+// the 31 updates of a 4096 x 4096 sweep: 55 us (40 TFLOP/s), 95 us as 64 x 64 tiles.
 __global__ void __launch_bounds__(256, 2)
 gptq_update_tiles_kernel(float* __restrict__ work, const float* __restrict__ deltas, const float* __restrict__ U,
                          int64_t rows, int64_t K, int start, int n, int end) {
