@@ -608,9 +608,9 @@ int vq_kivi_write_2bit(const void* in, void* scale, void* zero_point, void* pack
  * heads of the KV head); k_packed / v_packed: 2-bit codes [outer, Tm, 128] (four per byte); k_scale,
  * k_zero: bfloat16 [outer, Tm / k_block, 128]; v_scale, v_zero: bfloat16 [outer, Tm, 128 / v_block];
  * k_res, v_res: the newest R positions in bfloat16, [outer, R, 128].  VQ_EUNSUPPORTED unless D == 128,
- * G <= 8, k_block a multiple of 64 dividing Tm, v_block 32, 64 or 128, R a multiple of 16 and the
- * G * (Tm + R) * 6 bytes of scores fit in shared memory beside two staged chunks (G = 4: about 4600
- * positions) (the caller then reads the cache with
+ * G <= 8, k_block a multiple of 64 dividing Tm, v_block 32, 64 or 128, R 0 or at least 16 and the 6 bytes of score per query
+ * head and position of a CTA's share of the positions fit in shared memory beside two staged chunks (G = 4: about
+ * 4400 positions a share; up to eight CTAs share a pair's positions when there are few pairs) (the caller then reads the cache with
  * vq_kivi_read_2bit and runs the nodes one by one). */
 int vq_kivi_decode_attention(const void* q, const void* k_packed, const void* k_scale, const void* k_zero,
                              const void* v_packed, const void* v_scale, const void* v_zero, const void* k_res,
