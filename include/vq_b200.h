@@ -387,6 +387,13 @@ int vq_attention_fp8(const void* q8, const void* k8, const void* vt8, void* out8
                      int alpha_qk_dtype, float score_scale, const void* p_scale, int p_scale_dtype,
                      const void* alpha_pv, int alpha_pv_dtype, const void* ctx_scale, int ctx_scale_dtype,
                      int round_acc, void* stream);
+/* The same for any T: vt8's rows are ldv elements apart, ldv at least T and a multiple of 16 (what lies past T is not
+ * read). */
+int vq_attention_fp8_ragged(const void* q8, const void* k8, const void* vt8, int64_t ldv, void* out8, int64_t ld8,
+                            void* out16, int64_t T, int64_t kv_heads, int64_t groups, int64_t head_dim,
+                            const void* alpha_qk, int alpha_qk_dtype, float score_scale, const void* p_scale,
+                            int p_scale_dtype, const void* alpha_pv, int alpha_pv_dtype, const void* ctx_scale,
+                            int ctx_scale_dtype, int round_acc, void* stream);
 int vq_attention_status(int reset);
 
 /* Causal self-attention on bfloat16 operands in one kernel: the matmul / scale + mask / softmax /
@@ -404,6 +411,10 @@ int vq_attention_status(int reset);
 int vq_attention_bf16(const void* q, const void* k, const void* vt, void* out, int64_t ldo, int64_t T,
                       int64_t kv_heads, int64_t groups, int64_t head_dim, float score_scale, int round_acc,
                       void* stream);
+/* The same for any T: vt's rows are ldv elements apart, ldv at least T and a multiple of 8. */
+int vq_attention_bf16_ragged(const void* q, const void* k, const void* vt, int64_t ldv, void* out, int64_t ldo, int64_t T,
+                             int64_t kv_heads, int64_t groups, int64_t head_dim, float score_scale, int round_acc,
+                             void* stream);
 
 /* RMSNorm's backward of a training step: the input gradient (plus the residual stream's) and
  * the weight gradient from one read of the rows -- the operator
@@ -500,6 +511,11 @@ int vq_qkv_post_fp8(const void* q, const void* k, const void* v, int64_t ld, con
                     void* q_out, void* k_out, void* vt_out, int64_t T, int64_t q_heads, int64_t kv_heads, int64_t d,
                     const void* q_scale, int q_scale_dtype, const void* k_scale, int k_scale_dtype,
                     const void* v_scale, int v_scale_dtype, void* stream);
+/* The same with vt_out's rows vt_ld elements apart. */
+int vq_qkv_post_fp8_ragged(const void* q, const void* k, const void* v, int64_t ld, const void* cosv, const void* sinv,
+                           void* q_out, void* k_out, void* vt_out, int64_t vt_ld, int64_t T, int64_t q_heads,
+                           int64_t kv_heads, int64_t d, const void* q_scale, int q_scale_dtype, const void* k_scale,
+                           int k_scale_dtype, const void* v_scale, int v_scale_dtype, void* stream);
 int vq_transpose_quantize_fp8(const void* x, void* out, void* codes, void* amax_bits, int format, int64_t T,
                               int64_t heads, int64_t d, int64_t ldx, const void* scale, int scale_dtype,
                               void* stream);

@@ -137,6 +137,11 @@ SIGNATURES = {
     "vq_gemm_mx_rows_workspace_bytes": [_I64, _I64, _I64],
     "vq_gemm_mx_rows": [_P, _P, _P, _I, _P, _P, _P, _I64, _P, _I, _I64, _I64, _I64, _P, _I, _P, _I, _P, _P],
     "vq_gptq_factor": [_P, _P, _I64, _P, _P],
+    "vq_attention_fp8_ragged": [_P, _P, _P, _I64, _P, _I64, _P, _I64, _I64, _I64, _I64, _P, _I, _F, _P, _I, _P, _I, _P, _I,
+                                _I, _P],
+    "vq_attention_bf16_ragged": [_P, _P, _P, _I64, _P, _I64, _I64, _I64, _I64, _I64, _F, _I, _P],
+    "vq_qkv_post_fp8_ragged": [_P, _P, _P, _I64, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I64, _P, _I, _P, _I, _P, _I,
+                               _P],
     "vq_kivi_read_2bit": [_P, _P, _P, _P, _I64, _I64, _I64, _I, _I64, _P],
     "vq_gptq_block": [_P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I, _F, _F, _I, ctypes.POINTER(VqRound),
                       ctypes.POINTER(VqRound), _P],

@@ -181,7 +181,7 @@ template <bool E4M3>
 __device__ __forceinline__ void transpose_quantize_body(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ out,
                                                         uint8_t* __restrict__ codes, int* __restrict__ amax_bits, int T,
                                                         int heads, int d, int64_t ldx, const void* __restrict__ scale,
-                                                        int scale_dt, int bx, int by, int bz) {
+                                                        int scale_dt, int bx, int by, int bz, int64_t ldo) {
   __shared__ __align__(16) uint8_t tile[64][64 + 4];
   __shared__ int block_max;
   const Divisor dv = make_divisor(scale, scale_dt);
@@ -228,18 +228,18 @@ __device__ __forceinline__ void transpose_quantize_body(const __nv_bfloat16* __r
     for (int off = 16; off; off >>= 1) local_max = max(local_max, __shfl_xor_sync(0xFFFFFFFFu, local_max, off));
     if ((threadIdx.x & 31) == 0) atomicMax(&block_max, local_max);
   }
-  const bool wide = (T & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0;
+  const bool wide = ((T | ldo) & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0;
   if (wide) {
     for (int i = threadIdx.x; i < 64 * 16; i += blockDim.x) {
       const int jj = i >> 4, tq = (i & 15) << 2;
       if (t0 + tq < T && j0 + jj < d)   // T % 4 == 0: a group of four is inside or outside as a whole
-        *reinterpret_cast<uint32_t*>(out + ((int64_t)h * d + j0 + jj) * T + t0 + tq) =
+        *reinterpret_cast<uint32_t*>(out + ((int64_t)h * d + j0 + jj) * ldo + t0 + tq) =
             *reinterpret_cast<const uint32_t*>(&tile[jj][tq]);
     }
   } else {
     for (int i = threadIdx.x; i < 64 * 64; i += blockDim.x) {
       const int jj = i >> 6, tt = i & 63;
-      if (t0 + tt < T && j0 + jj < d) out[((int64_t)h * d + j0 + jj) * T + t0 + tt] = tile[jj][tt];
+      if (t0 + tt < T && j0 + jj < d) out[((int64_t)h * d + j0 + jj) * ldo + t0 + tt] = tile[jj][tt];
     }
   }
   if (amax_bits != nullptr) {
@@ -253,7 +253,7 @@ transpose_quantize_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restri
                           int* __restrict__ amax_bits, int T, int heads, int d, int64_t ldx,
                           const void* __restrict__ scale, int scale_dt) {
   transpose_quantize_body<E4M3>(x, out, codes, amax_bits, T, heads, d, ldx, scale, scale_dt, (int)blockIdx.x,
-                                (int)blockIdx.y, (int)blockIdx.z);
+                                (int)blockIdx.y, (int)blockIdx.z, T);
 }
 
 // The three casts between the merged q/k/v projection and the attention kernel as one launch: RoPE + cast of the
@@ -265,6 +265,7 @@ struct QkvPostParams {
   uint2 *q_out, *k_out;
   uint8_t* vt_out;
   int T, q_heads, kv_heads, d;
+  int64_t vt_ld;            // elements between the rows of vt_out
   int64_t ld;               // elements between consecutive tokens of q, k and v (slices of one [T, *] matrix)
   const void *q_scale, *k_scale, *v_scale;
   int q_scale_dt, k_scale_dt, v_scale_dt;
@@ -285,7 +286,7 @@ qkv_post_kernel(const QkvPostParams p) {
     const int per_head = p.v_tiles_t * p.v_tiles_d;
     const int h = i / per_head, rem = i - h * per_head;
     transpose_quantize_body<true>(p.v, p.vt_out, nullptr, nullptr, p.T, p.kv_heads, p.d, p.ld, p.v_scale, p.v_scale_dt,
-                                  rem % p.v_tiles_t, rem / p.v_tiles_t, h);
+                                  rem % p.v_tiles_t, rem / p.v_tiles_t, h, p.vt_ld);
   }
 }
 
@@ -598,6 +599,16 @@ extern "C" int vq_qkv_post_fp8(const void* q, const void* k, const void* v, int6
                                void* q_out, void* k_out, void* vt_out, int64_t T, int64_t q_heads, int64_t kv_heads,
                                int64_t d, const void* q_scale, int q_scale_dtype, const void* k_scale,
                                int k_scale_dtype, const void* v_scale, int v_scale_dtype, void* stream) {
+  return vq_qkv_post_fp8_ragged(q, k, v, ld, cosv, sinv, q_out, k_out, vt_out, T, T, q_heads, kv_heads, d, q_scale,
+                                q_scale_dtype, k_scale, k_scale_dtype, v_scale, v_scale_dtype, stream);
+}
+
+extern "C" int vq_qkv_post_fp8_ragged(const void* q, const void* k, const void* v, int64_t ld, const void* cosv,
+                                      const void* sinv, void* q_out, void* k_out, void* vt_out, int64_t vt_ld, int64_t T,
+                                      int64_t q_heads, int64_t kv_heads, int64_t d, const void* q_scale,
+                                      int q_scale_dtype, const void* k_scale, int k_scale_dtype, const void* v_scale,
+                                      int v_scale_dtype, void* stream) {
+  VQ_REQUIRE(vt_ld >= T, "vq_qkv_post_fp8: the values' row stride is smaller than a row");
   VQ_REQUIRE(T >= 0 && q_heads >= 0 && kv_heads >= 0 && d >= 0, "vq_qkv_post_fp8: bad extent");
   if (T == 0 || d == 0 || (q_heads == 0 && kv_heads == 0)) return VQ_OK;
   VQ_REQUIRE(q && k && v && cosv && sinv && q_out && k_out && vt_out && q_scale && k_scale && v_scale,
@@ -612,7 +623,7 @@ extern "C" int vq_qkv_post_fp8(const void* q, const void* k, const void* v, int6
   p.q = static_cast<const uint4*>(q); p.k = static_cast<const uint4*>(k); p.v = static_cast<const __nv_bfloat16*>(v);
   p.cosv = static_cast<const uint4*>(cosv); p.sinv = static_cast<const uint4*>(sinv);
   p.q_out = static_cast<uint2*>(q_out); p.k_out = static_cast<uint2*>(k_out); p.vt_out = static_cast<uint8_t*>(vt_out);
-  p.T = (int)T; p.q_heads = (int)q_heads; p.kv_heads = (int)kv_heads; p.d = (int)d; p.ld = ld;
+  p.T = (int)T; p.q_heads = (int)q_heads; p.kv_heads = (int)kv_heads; p.d = (int)d; p.ld = ld; p.vt_ld = vt_ld;
   p.q_scale = q_scale; p.k_scale = k_scale; p.v_scale = v_scale;
   p.q_scale_dt = q_scale_dtype; p.k_scale_dt = k_scale_dtype; p.v_scale_dt = v_scale_dtype;
   // the rope jobs get blocks in proportion to their elements, about eight blocks per SM in all

@@ -148,10 +148,24 @@ def softmax_quantize_fp8(scores: torch.Tensor, score_scale: float, out_scale: to
     return out
 
 
+def _value_rows(vt: torch.Tensor):
+    """``vt [kv, 128, T]`` as ``(tensor, row stride)`` with the row stride a multiple of 16 bytes: as it stands, or copied
+    into padded rows."""
+    kv, d, T = vt.shape
+    step = 16 // vt.element_size()
+    ld = vt.stride(1)
+    if vt.stride(2) == 1 and ld >= T and ld % step == 0 and vt.stride(0) == d * ld and vt.data_ptr() % 16 == 0:
+        return vt, ld
+    ld = -(-T // step) * step
+    rows = torch.empty((kv, d, ld), dtype=vt.dtype, device=vt.device)
+    rows[:, :, :T].copy_(vt)
+    return rows, ld
+
+
 @N.device_guarded
 def attention_fp8(q8: torch.Tensor, k8: torch.Tensor, vt8: torch.Tensor, alpha_qk: torch.Tensor, score_scale: float,
                   p_scale: torch.Tensor, alpha_pv: torch.Tensor, ctx_scale: Optional[torch.Tensor] = None,
-                  round_acc: bool = False):
+                  round_acc: bool = False, ragged: bool = False):
     """Causal attention on FP8 operands in one kernel: ``fp8_gemm(q8, k8, alpha_qk)``,
     ``softmax_quantize_fp8(.., score_scale, p_scale, causal_period=T)``, ``fp8_gemm(p8, vt8, alpha_pv)``
     and, with ``ctx_scale``, the cast of the context, with the same rounding steps.
@@ -159,13 +173,14 @@ def attention_fp8(q8: torch.Tensor, k8: torch.Tensor, vt8: torch.Tensor, alpha_q
     ``k8``: ``[kv_heads, T, 128]``, ``vt8``: ``[kv_heads, 128, T]``, all e4m3 codes.
     Returns the e4m3 context ``[T, heads * 128]`` when ``ctx_scale`` is given, else the
     bfloat16 context ``[kv_heads, groups * T, 128]``.  ``round_acc``: both GEMMs as
-    ``fp8_gemm(..., round_acc=True)``."""
+    ``fp8_gemm(..., round_acc=True)``.  ``T`` is a multiple of 128 unless ``ragged`` says that it may be any."""
     kv, rows, d = q8.shape
     T = k8.shape[1]
     groups = rows // T
     if k8.shape != (kv, T, d) or vt8.shape != (kv, d, T) or groups * T != rows:
         raise ValueError("attention_fp8: operand shapes do not agree")
-    q8, k8, vt8 = q8.contiguous(), k8.contiguous(), vt8.contiguous()
+    q8, k8 = q8.contiguous(), k8.contiguous()
+    vt8, ldv = _value_rows(vt8) if ragged else (vt8.contiguous(), T)
     scalars = [_scale_arg(t) for t in (alpha_qk, p_scale, alpha_pv)]
     out8 = out16 = None
     if ctx_scale is not None:
@@ -173,13 +188,15 @@ def attention_fp8(q8: torch.Tensor, k8: torch.Tensor, vt8: torch.Tensor, alpha_q
         out8 = torch.empty((T, kv * groups * d), dtype=torch.uint8, device=q8.device)
     else:
         out16 = torch.empty((kv, rows, d), dtype=torch.bfloat16, device=q8.device)
-    N.check(N.lib().vq_attention_fp8(q8.data_ptr(), k8.data_ptr(), vt8.data_ptr(), _ptr(out8), kv * groups * d,
-                                     _ptr(out16), T, kv, groups, d, scalars[0].data_ptr(), _dtype_id(scalars[0].dtype),
-                                     float(score_scale), scalars[1].data_ptr(), _dtype_id(scalars[1].dtype),
-                                     scalars[2].data_ptr(), _dtype_id(scalars[2].dtype), _ptr(ctx_scale),
-                                     _dtype_id(ctx_scale.dtype) if ctx_scale is not None else 0, int(bool(round_acc)),
-                                     _stream()),
-            "vq_attention_fp8")
+    rest = (_ptr(out8), kv * groups * d, _ptr(out16), T, kv, groups, d, scalars[0].data_ptr(), _dtype_id(scalars[0].dtype),
+            float(score_scale), scalars[1].data_ptr(), _dtype_id(scalars[1].dtype), scalars[2].data_ptr(),
+            _dtype_id(scalars[2].dtype), _ptr(ctx_scale), _dtype_id(ctx_scale.dtype) if ctx_scale is not None else 0,
+            int(bool(round_acc)), _stream())
+    if ragged:
+        N.check(N.lib().vq_attention_fp8_ragged(q8.data_ptr(), k8.data_ptr(), vt8.data_ptr(), ldv, *rest),
+                "vq_attention_fp8_ragged")
+    else:
+        N.check(N.lib().vq_attention_fp8(q8.data_ptr(), k8.data_ptr(), vt8.data_ptr(), *rest), "vq_attention_fp8")
     return out8 if out8 is not None else out16
 
 
@@ -220,18 +237,26 @@ def rope_heads_bf16(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> to
 
 @N.device_guarded
 def attention_bf16_heads(q_heads: torch.Tensor, k_heads: torch.Tensor, vt: torch.Tensor,
-                         score_scale: Optional[float] = None, round_acc: bool = True) -> torch.Tensor:
+                         score_scale: Optional[float] = None, round_acc: bool = True,
+                         ragged: bool = False) -> torch.Tensor:
     """``attention_bf16`` on operands already in the kernel's layout: ``q_heads [heads, T, 128]``, ``k_heads
-    [kv_heads, T, 128]`` (what ``rope_heads_bf16`` writes) and ``vt [kv_heads, 128, T]`` -> ``[T, heads * 128]``."""
+    [kv_heads, T, 128]`` (what ``rope_heads_bf16`` writes) and ``vt [kv_heads, 128, T]`` -> ``[T, heads * 128]``.
+    ``T`` is a multiple of 128 unless ``ragged`` says that it may be any."""
     heads, T, d = q_heads.shape
     kv = k_heads.shape[0]
     if k_heads.shape != (kv, T, d) or vt.shape != (kv, d, T) or heads % kv:
         raise ValueError("attention_bf16_heads: operand shapes do not agree")
     if any(t.dtype != torch.bfloat16 for t in (q_heads, k_heads, vt)):
         raise NotImplementedError("attention_bf16_heads takes bfloat16 operands")
-    q_heads, k_heads, vt = q_heads.contiguous(), k_heads.contiguous(), vt.contiguous()
+    q_heads, k_heads = q_heads.contiguous(), k_heads.contiguous()
+    vt, ldv = _value_rows(vt) if ragged else (vt.contiguous(), T)
     out = torch.empty((T, heads * d), dtype=torch.bfloat16, device=q_heads.device)
     scale = 1.0 / math.sqrt(d) if score_scale is None else float(score_scale)
+    if ragged:
+        N.check(N.lib().vq_attention_bf16_ragged(q_heads.data_ptr(), k_heads.data_ptr(), vt.data_ptr(), ldv, out.data_ptr(),
+                                                 heads * d, T, kv, heads // kv, d, scale, int(bool(round_acc)),
+                                                 _stream()), "vq_attention_bf16_ragged")
+        return out
     N.check(N.lib().vq_attention_bf16(q_heads.data_ptr(), k_heads.data_ptr(), vt.data_ptr(), out.data_ptr(), heads * d, T,
                                       kv, heads // kv, d, scale, int(bool(round_acc)), _stream()), "vq_attention_bf16")
     return out
@@ -359,11 +384,12 @@ def rope_quantize_fp8(x: torch.Tensor, cos: Optional[torch.Tensor], sin: Optiona
 
 @N.device_guarded
 def qkv_post_fp8(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
-                 q_scale: torch.Tensor, k_scale: torch.Tensor, v_scale: torch.Tensor):
+                 q_scale: torch.Tensor, k_scale: torch.Tensor, v_scale: torch.Tensor, ragged: bool = False):
     """``rope_quantize_fp8(q)``, ``rope_quantize_fp8(k)`` and ``transpose_quantize_fp8(v)`` as one launch, for
     ``q [T, heads, d]``, ``k`` / ``v [T, kv_heads, d]`` that are column slices of one ``[T, *]`` matrix (the output
     of a merged q/k/v projection).  Returns ``(q8 [heads, T, d], k8 [kv_heads, T, d], vt8 [kv_heads, d, T])``, equal
-    to the separate calls bit for bit; operands that are not such slices take the separate calls."""
+    to the separate calls bit for bit; operands that are not such slices take the separate calls.  ``ragged``: ``vt8``'s
+    rows may be padded to a multiple of 16 bytes, as ``attention_fp8(ragged=True)`` reads them."""
     T, heads, d = q.shape
     kv = k.shape[1]
     views = [_heads_view("qkv_post_fp8", t) for t in (q, k, v)]
@@ -377,13 +403,13 @@ def qkv_post_fp8(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.T
     scales = [_scale_arg(t) for t in (q_scale, k_scale, v_scale)]
     q8 = torch.empty((heads, T, d), dtype=torch.uint8, device=q.device)
     k8 = torch.empty((kv, T, d), dtype=torch.uint8, device=q.device)
-    vt8 = torch.empty((kv, d, T), dtype=torch.uint8, device=q.device)
-    N.check(N.lib().vq_qkv_post_fp8(q.data_ptr(), k.data_ptr(), v.data_ptr(), views[0][1], cos.data_ptr(), sin.data_ptr(),
-                                    q8.data_ptr(), k8.data_ptr(), vt8.data_ptr(), T, heads, kv, d,
-                                    scales[0].data_ptr(), _dtype_id(scales[0].dtype), scales[1].data_ptr(),
-                                    _dtype_id(scales[1].dtype), scales[2].data_ptr(), _dtype_id(scales[2].dtype), _stream()),
-            "vq_qkv_post_fp8")
-    return q8, k8, vt8
+    ldv = -(-T // 16) * 16 if ragged else T
+    vt8 = torch.empty((kv, d, ldv), dtype=torch.uint8, device=q.device)
+    N.check(N.lib().vq_qkv_post_fp8_ragged(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), views[0][1], cos.data_ptr(), sin.data_ptr(), q8.data_ptr(), k8.data_ptr(),
+        vt8.data_ptr(), ldv, T, heads, kv, d, scales[0].data_ptr(), _dtype_id(scales[0].dtype), scales[1].data_ptr(),
+        _dtype_id(scales[1].dtype), scales[2].data_ptr(), _dtype_id(scales[2].dtype), _stream()), "vq_qkv_post_fp8")
+    return q8, k8, vt8 if ldv == T else vt8[:, :, :T]
 
 
 @N.device_guarded

@@ -204,7 +204,7 @@ class Fp8DecoderLayer:
         # query heads of one KV group are stacked along the rows: [kv, groups*T, d]
         if self.merge_qkv:
             # slices of one matrix: the two RoPE casts and the value transpose are one launch
-            q8, k8, vt8 = FP8.qkv_post_fp8(q, k, v, cos, sin, s["q"], s["k"], s["v"])
+            q8, k8, vt8 = FP8.qkv_post_fp8(q, k, v, cos, sin, s["q"], s["k"], s["v"], ragged=self.fuse_attention)
             q8 = q8.view(sh.kv_heads, sh.groups * T, sh.head_dim)
         else:
             # the small K and V casts run beside the Q cast on a second stream (a fork and join that a
@@ -221,9 +221,9 @@ class Fp8DecoderLayer:
             for t in (k8, vt8):
                 t.record_stream(main)
             k.record_stream(self._side)
-        if self.fuse_attention and T % 128 == 0:
+        if self.fuse_attention:
             ctx8 = FP8.attention_fp8(q8, k8, vt8, self.alpha_qk, 1.0 / math.sqrt(sh.head_dim), s["p"], self.alpha_pv,
-                                     s["ctx"], round_acc=self.ra)            # [T, heads*d]
+                                     s["ctx"], round_acc=self.ra, ragged=True)   # [T, heads*d]
             return self._after_attention(x, ctx8)
         # masked scores are neither computed nor read; masked probabilities are zero codes
         scores = FP8.fp8_gemm(q8, k8, self.alpha_qk, causal=("scores", T), round_acc=self.ra)  # [kv, groups*T, T]
@@ -308,7 +308,7 @@ class Nvfp4DecoderLayer:
         self.NV, self.shape, self.merge = NV, shape, merge
         # "eager": the graph's own attention operators (matmul, scale + mask, softmax, matmul: HF eager
         # attention, every intermediate a bfloat16 tensor).  "fused": the same roundings inside this package's
-        # one-kernel attention (head_dim 128, T a multiple of 128; other shapes run "eager").  "sdpa": torch's
+        # one-kernel attention (head_dim 128; other shapes run "eager").  "sdpa": torch's
         # fused kernel, which keeps the scores in float32; it differs from the other two by the bfloat16
         # rounding of the scores (half a unit at 64..128), which the 4-bit casts downstream amplify to
         # quantization-noise level.
@@ -380,14 +380,14 @@ class Nvfp4DecoderLayer:
         cos, sin = self._rope
         h = F.rms_norm(x, (sh.hidden,), self.ln1, sh.eps)
         q, k, v = self._linear(h, ("q", "k", "v"))
-        if self.attention == "fused" and sh.head_dim == 128 and T % 128 == 0:
+        if self.attention == "fused" and sh.head_dim == 128:
             # RoPE straight into the attention kernel's head-major layout (slices of the merged projection are
             # read in place), V transposed for the P V contraction
             from . import fp8 as F8
 
             ctx = F8.attention_bf16_heads(F8.rope_heads_bf16(q.unflatten(1, (sh.heads, sh.head_dim)), cos, sin),
                                           F8.rope_heads_bf16(k.unflatten(1, (sh.kv_heads, sh.head_dim)), cos, sin),
-                                          v.unflatten(1, (sh.kv_heads, sh.head_dim)).permute(1, 2, 0).contiguous())
+                                          v.unflatten(1, (sh.kv_heads, sh.head_dim)).permute(1, 2, 0), ragged=True)
         else:
             q = apply_rope(q.reshape(T, sh.heads, sh.head_dim), cos, sin)
             k = apply_rope(k.reshape(T, sh.kv_heads, sh.head_dim), cos, sin)
