@@ -65,7 +65,9 @@ typedef struct VqRound {
   const void* steps;
   uint16_t nan_value;
   /* SEARCH / STOCHASTIC: device float arrays */
-  const float* edges;     /* SEARCH: ascending edges, result = #edges < v */
+  const float* edges;     /* SEARCH: ascending edges, result = #edges < v.  TABLE (optional, n_edges 1 to 15; HOST
+                             memory, copied by the call): ascending bfloat16 values, the table's entry for v being
+                             #edges <= v for every v that is no NaN */
   const float* levels;    /* SEARCH (optional: value per index) / STOCHASTIC */
   int32_t n_edges;
   int32_t n_levels;

@@ -190,3 +190,23 @@ def test_convolution_operator_schemas_are_the_references():
     y = Q.conv2d(x.permute(0, 2, 3, 1), w.permute(2, 3, 1, 0), None, [2, 2], [1, 1], [1, 1], 1, layout="nhwc",
                  out_dtype=torch.float32)
     assert y.shape == (2, 5, 5, 8) and y.dtype == torch.float32
+
+
+def test_index_tables_are_counts_of_edges():
+    """The edges found for an index table give every entry back; tables of another kind have none."""
+    R = voyager_b200.rounding
+    patterns = np.arange(1 << 16, dtype=np.uint32)
+    x = (patterns << 16).view(np.float32)
+    idx, levels = voyager_b200.formats.index_table(voyager_b200.get_quantization_map("lut4_to_int6"))
+    bits = idx.to(torch.bfloat16).view(torch.int16).numpy().view(np.uint16)
+    edges = R._count_edges(bits)
+    assert edges.size == levels.numel() - 1
+    counts = (x[:, None] >= edges[None, :]).sum(1).astype(np.float32)
+    entries = (bits.astype(np.uint32) << 16).view(np.float32)
+    assert np.array_equal(counts[~np.isnan(x)], entries[~np.isnan(x)])
+    for name in ("posit8_1", "int8", "fp8_e4m3", "uint8"):
+        assert R._count_edges(voyager_b200.formats._table_bits(name)) is None, name
+    step = np.where(x >= 0, 0x3F80, 0).astype(np.uint16)         # 1 from -0 on: a comparison with -0 sees both zeros
+    assert R._count_edges(step).size == 1
+    step[0x8000] = 0                                             # 1 from +0 on: no comparison tells it from -0
+    assert R._count_edges(step) is None

@@ -256,6 +256,109 @@ transpose_quantize_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restri
                                 (int)blockIdx.y, (int)blockIdx.z, T);
 }
 
+__device__ __noinline__ uint4 quotients8_exact(uint4 x, float s) {
+  const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(__fdiv_rn(lo_of(w[j]), s), __fdiv_rn(hi_of(w[j]), s));
+    o[j] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// The same cast and transpose for whole 16-byte pieces: 128 x 128 tiles, 512 threads of four rows x eight columns.  A
+// thread's four loads are independent; the eight quotients of a row share one test for a nearby bfloat16 midpoint
+// (quotients too small for its argument cast to a zero of their sign either way); 4 x 4 bytes are transposed in registers
+// and go to shared memory as words, exclusive-ored so that a warp's stores and 16-byte reads touch every bank once.
+// 4096 x 4096 with both outputs and the maximum (64 MB): 17.5 us, 25.7 as 64 x 64 tiles with a byte store per element.
+template <bool E4M3>
+__global__ void __launch_bounds__(512, 2)
+cast_transpose_kernel(const uint4* __restrict__ x, uint8_t* __restrict__ out, uint8_t* __restrict__ codes,
+                      int* __restrict__ amax_bits, int T, int heads, int d, int64_t ldx, const void* __restrict__ scale,
+                      int scale_dt) {
+  __shared__ __align__(16) uint32_t tile[128][32];   // column j's codes of 128 rows; word w stands at w ^ (j / 8 % 16 * 2)
+  __shared__ int block_max;
+  const Divisor dv = make_divisor(scale, scale_dt);
+  const int h = blockIdx.z, t0 = blockIdx.x * 128, j0 = blockIdx.y * 128;
+  const int v = threadIdx.x & 15, tq = threadIdx.x >> 4;
+  const bool inside = j0 + v * 8 < d;   // d % 8 == 0: a vector is inside or outside as a whole
+  if (threadIdx.x == 0) block_max = 0;
+  __syncthreads();
+  uint4 r[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    r[i] = make_uint4(0, 0, 0, 0);
+    const int t = t0 + tq * 4 + i;
+    if (t < T && inside) r[i] = __ldg(x + ((int64_t)t * ldx + (int64_t)h * d + j0) / 8 + v);
+  }
+  uint32_t lo[4], hi[4], m = 0;   // codes of columns 0..3 and 4..7 of each row
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint32_t w[4] = {r[i].x, r[i].y, r[i].z, r[i].w}, near = 0xFFFFFFFFu;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      m = __vmaxu2(m, w[j] & 0x7FFF7FFFu);
+      const float a = __fmul_rn(lo_of(w[j]), dv.rcp), b = __fmul_rn(hi_of(w[j]), dv.rcp);
+      near = min(near, min(__float_as_uint(a) * 65536u - 0x7FFD0000u, __float_as_uint(b) * 65536u - 0x7FFD0000u));
+      const __nv_bfloat162 q = __floats2bfloat162_rn(a, b);
+      w[j] = *reinterpret_cast<const uint32_t*>(&q);
+    }
+    if (near <= 0x0006FFFFu || !dv.ordinary) {
+      const uint4 e = quotients8_exact(r[i], dv.s);
+      w[0] = e.x; w[1] = e.y; w[2] = e.z; w[3] = e.w;
+    }
+    lo[i] = fp8_pair<E4M3>(lo_of(w[0]), hi_of(w[0])) | (fp8_pair<E4M3>(lo_of(w[1]), hi_of(w[1])) << 16);
+    hi[i] = fp8_pair<E4M3>(lo_of(w[2]), hi_of(w[2])) | (fp8_pair<E4M3>(lo_of(w[3]), hi_of(w[3])) << 16);
+    const int t = t0 + tq * 4 + i;
+    if (codes != nullptr && t < T && inside)
+      *reinterpret_cast<uint2*>(codes + ((int64_t)t * heads + h) * d + j0 + v * 8) = make_uint2(lo[i], hi[i]);
+  }
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const uint32_t a = half ? hi[0] : lo[0], b = half ? hi[1] : lo[1], c = half ? hi[2] : lo[2], e = half ? hi[3] : lo[3];
+    const uint32_t ab0 = __byte_perm(a, b, 0x5140), ab1 = __byte_perm(a, b, 0x7362);   // a0 b0 a1 b1, a2 b2 a3 b3
+    const uint32_t ce0 = __byte_perm(c, e, 0x5140), ce1 = __byte_perm(c, e, 0x7362);
+    uint32_t (*col)[32] = tile + v * 8 + half * 4;
+    const int at = tq ^ (2 * v);
+    col[0][at] = __byte_perm(ab0, ce0, 0x5410);
+    col[1][at] = __byte_perm(ab0, ce0, 0x7632);
+    col[2][at] = __byte_perm(ab1, ce1, 0x5410);
+    col[3][at] = __byte_perm(ab1, ce1, 0x7632);
+  }
+  if (amax_bits != nullptr) {
+    int local = (int)max(m & 0xFFFFu, m >> 16);
+    for (int off = 16; off; off >>= 1) local = max(local, __shfl_xor_sync(0xFFFFFFFFu, local, off));
+    if ((threadIdx.x & 31) == 0) atomicMax(&block_max, local);
+  }
+  __syncthreads();
+  const int piece = threadIdx.x & 7;   // 16 bytes of a column
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int j = (threadIdx.x >> 3) + 64 * u, s = (j >> 3) * 2;
+    if (j0 + j >= d) continue;
+    uint4 c = *reinterpret_cast<const uint4*>(&tile[j][4 * (piece ^ (s >> 2))]);
+    if (s & 2) c = make_uint4(c.z, c.w, c.x, c.y);
+    const int t = t0 + piece * 16;
+    uint8_t* dst = out + ((int64_t)h * d + j0 + j) * T + t;
+    if ((T & 15) == 0) {
+      if (t < T) *reinterpret_cast<uint4*>(dst) = c;
+    } else {
+      const uint32_t w[4] = {c.x, c.y, c.z, c.w};
+      if ((T & 3) == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (t + 4 * q < T) reinterpret_cast<uint32_t*>(dst)[q] = w[q];
+      } else {
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+          if (t + q < T) dst[q] = (uint8_t)(w[q >> 2] >> (8 * (q & 3)));
+      }
+    }
+  }
+  if (amax_bits != nullptr && threadIdx.x == 0) atomicMax(amax_bits, block_max);
+}
+
 // The three casts between the merged q/k/v projection and the attention kernel as one launch: RoPE + cast of the
 // query heads and of the key heads (head-major outputs), cast + transpose of the value heads.  Blocks
 // [0, q_blocks) take the queries, the next k_blocks the keys, the rest one value tile each.
@@ -646,8 +749,21 @@ extern "C" int vq_transpose_quantize_fp8(const void* x, void* out, void* codes, 
   VQ_REQUIRE(format == VQ_IN_E4M3 || format == VQ_IN_E5M2, "vq_transpose_quantize_fp8: format must be e4m3 or e5m2");
   VQ_REQUIRE(T < (1ll << 31) && heads < 65536 && d < (1 << 22), "vq_transpose_quantize_fp8: extent too large");
   VQ_REQUIRE(ldx >= heads * d, "vq_transpose_quantize_fp8: row stride smaller than a row");
-  dim3 grid((unsigned)((T + 63) / 64), (unsigned)((d + 63) / 64), (unsigned)heads);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (d % 8 == 0 && ldx % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
+      (reinterpret_cast<uintptr_t>(codes) & 7) == 0) {
+    const dim3 tiles((unsigned)((T + 127) / 128), (unsigned)((d + 127) / 128), (unsigned)heads);
+    if (format == VQ_IN_E4M3)
+      cast_transpose_kernel<true><<<tiles, 512, 0, st>>>(static_cast<const uint4*>(x), static_cast<uint8_t*>(out),
+                                                         static_cast<uint8_t*>(codes), static_cast<int*>(amax_bits), (int)T,
+                                                         (int)heads, (int)d, ldx, scale, scale_dtype);
+    else
+      cast_transpose_kernel<false><<<tiles, 512, 0, st>>>(static_cast<const uint4*>(x), static_cast<uint8_t*>(out),
+                                                          static_cast<uint8_t*>(codes), static_cast<int*>(amax_bits),
+                                                          (int)T, (int)heads, (int)d, ldx, scale, scale_dtype);
+    return check_launch("cast_transpose_kernel");
+  }
+  dim3 grid((unsigned)((T + 63) / 64), (unsigned)((d + 63) / 64), (unsigned)heads);
   if (format == VQ_IN_E4M3)
     transpose_quantize_kernel<true><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(out),
                                                           static_cast<uint8_t*>(codes), static_cast<int*>(amax_bits),

@@ -8,6 +8,7 @@
 
 #include <cstdarg>
 #include <cstdio>
+#include <cstring>
 
 #include "../../include/vq_b200.h"
 
@@ -95,6 +96,8 @@ struct Round {
   const uint16_t* steps;  // n_steps keys then n_steps values (global or shared)
   int32_t n_steps;
   uint32_t nan_value;
+  int32_t n_count;        // TABLE: how many of `count` there are, 0 if the table is no index table of 16 entries or fewer
+  uint16_t count[15];     // ascending bfloat16 values: the entry for v is how many of them v reaches; NaN past the last
 };
 
 inline Round make_round(const VqRound* r) {
@@ -119,6 +122,16 @@ inline Round make_round(const VqRound* r) {
   d.steps = static_cast<const uint16_t*>(r->steps);
   d.n_steps = r->n_steps;
   d.nan_value = r->nan_value;
+  if (r->mode == VQ_ROUND_TABLE && r->edges != nullptr && r->n_edges >= 1 && r->n_edges <= 15) {
+    d.edges = nullptr;    // host memory
+    d.n_edges = 0;
+    d.n_count = r->n_edges;
+    for (int i = 0; i < 15; ++i) {
+      uint32_t bits = 0x7FC00000u;
+      if (i < r->n_edges) memcpy(&bits, r->edges + i, sizeof(bits));
+      d.count[i] = (uint16_t)(bits >> 16);
+    }
+  }
   return d;
 }
 

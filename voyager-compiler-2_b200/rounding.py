@@ -12,6 +12,7 @@ else is gathered.
 """
 
 import ctypes
+import functools
 import hashlib
 import math
 
@@ -86,6 +87,30 @@ def _steps_of(bits: np.ndarray):
     return values.astype(np.uint16), uppers.astype(np.uint16), int(nan_entries[0])
 
 
+@functools.lru_cache(maxsize=1)
+def _value_order():
+    """The non-NaN bfloat16 patterns in the order of their values (-0 before +0), and the position of +0."""
+    patterns = np.arange(1 << 16, dtype=np.int64)
+    patterns = patterns[(patterns & 0x7FFF) <= 0x7F80]
+    order = patterns[np.argsort(_ordered_key(patterns), kind="stable")]
+    return order, int(np.flatnonzero(order == 0)[0])
+
+
+def _count_edges(bits: np.ndarray):
+    """The ascending bfloat16 values ``e`` of an index table whose entry for every non-NaN input ``x`` is the number of
+    ``e <= x`` (a lookup format's index table), at most 15 of them, as float32; ``None`` for any other table."""
+    order, zero = _value_order()
+    entries = bits[order]
+    starts = np.flatnonzero(entries[1:] != entries[:-1]) + 1
+    # runs 0, 1, 2, ...; no run begins at +0, which a comparison does not tell from -0
+    if not 1 <= starts.size <= 15 or entries[0] != 0 or zero in starts:
+        return None
+    counts = (entries[starts].astype(np.uint32) << 16).view(np.float32)
+    if not np.array_equal(counts, np.arange(1, starts.size + 1, dtype=np.float32)):
+        return None
+    return np.ascontiguousarray((order[starts].astype(np.uint32) << 16).view(np.float32))
+
+
 class RoundSpec:
     """A ``VqRound`` plus the tensors it points into (kept alive with it)."""
 
@@ -110,6 +135,7 @@ def none_round() -> RoundSpec:
 
 _NONE = None
 _table_cache = {}
+_edges_by_content = {}   # digest of a table's entries -> its edges or None
 
 
 def _classify_table(table_bf16: torch.Tensor, allow_arithmetic=True) -> RoundSpec:
@@ -119,7 +145,8 @@ def _classify_table(table_bf16: torch.Tensor, allow_arithmetic=True) -> RoundSpe
     if not allow_arithmetic:
         return RoundSpec(c, (table_bf16,))
     bits = table_bf16.view(torch.int16).cpu().numpy().view(np.uint16)
-    name = _canonical_fingerprints().get(_digest(bits))
+    digest = _digest(bits)
+    name = _canonical_fingerprints().get(digest)
     if name is not None:
         if (r := formats.int_range(name)) is not None:
             c.mode = N.ROUND_INT
@@ -133,6 +160,18 @@ def _classify_table(table_bf16: torch.Tensor, allow_arithmetic=True) -> RoundSpe
             c.is_signed = int(fmt.signed)
             return RoundSpec(c, (table_bf16,))
     steps = _steps_of(bits) if PREFER_STEPS else None
+    edges = None
+    if steps is None:
+        if digest not in _edges_by_content:
+            if len(_edges_by_content) > 64:
+                _edges_by_content.clear()
+            _edges_by_content[digest] = _count_edges(bits)
+        edges = _edges_by_content[digest]
+    if edges is not None:
+        # an index table: beside the table, the kernels get the edges to count, by value (a captured launch keeps them)
+        c.edges = edges.ctypes.data
+        c.n_edges = edges.size
+        return RoundSpec(c, (table_bf16, edges))
     if steps is not None:
         values, uppers, nan_value = steps
         packed = np.concatenate([uppers, values]).astype(np.uint16).view(np.int16)
