@@ -646,8 +646,8 @@ int vq_kivi_decode_attention(const void* q, const void* k_packed, const void* k_
  * (n_a_levels bfloat16 entries) is given; a_scale [M, K / block_size] may be NULL.
  * K is a multiple of 128; block_size a multiple of 32 dividing K.  workspace is
  * vq_gemm_lut4_workspace_floats(M, N, K) floats of device scratch (contents irrelevant);
- * counters is vq_gemm_lut4_counters(N) ints that must be zero before the first call and are
- * left zero by every call (calls sharing them must not overlap on the device). */
+ * counters is vq_gemm_lut4_counters(N) ints, cleared by every call (calls sharing them, or the
+ * workspace, must not overlap on the device). */
 int64_t vq_gemm_lut4_workspace_floats(int64_t M, int64_t N, int64_t K);
 int64_t vq_gemm_lut4_counters(int64_t N);
 int vq_gemm_lut4(const void* a, int64_t lda, const void* a_scale, const void* a_levels, int n_a_levels, int64_t M,

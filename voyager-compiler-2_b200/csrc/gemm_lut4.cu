@@ -82,7 +82,7 @@ struct Lut4Params {
   const void* bias;
   int bias_dt;
   float* workspace;         // [tiles][max_parts][accumulators of a tile]
-  int* counters;            // [tiles], zero between launches
+  int* counters;            // [tiles], cleared before each launch
   int tiles;                // row tiles
   int steps;                // K / step
   int slices;               // K slices: slice s holds steps s * steps / slices .. (s + 1) * steps / slices
@@ -433,7 +433,6 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       for (int q = 0; q < parts; ++q)
 #pragma unroll
         for (int e = 0; e < E; ++e) acc[e / (NT * 4)][(e / 4) % NT][e % 4] += __ldcg(slots + (int64_t)q * (E * 32) + e * 32);
-      if (lane == 0) p.counters[tile] = 0;   // ready for the next launch
     }
     output(tile);
   };
@@ -636,6 +635,9 @@ static int launch_row_stream(Lut4Params p, cudaStream_t st) {
     cudaFuncSetAttribute(gemm_lut4_kernel<WIDE, 3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
     cudaFuncSetAttribute(gemm_lut4_kernel<WIDE, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
   }
+  // cleared by every call and not by the last launch's tiles: a launch that gave up leaves some of them counted in part
+  if (cudaMemsetAsync(p.counters, 0, (size_t)q.tiles * sizeof(int), st) != cudaSuccess)
+    return fail(VQ_ECUDA, "row stream: memset");
   const dim3 grid((unsigned)q.ctas, (unsigned)q.slices);
   if (q.nt == 1) gemm_lut4_kernel<WIDE, 1, 4><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
   else if (q.nt == 2) gemm_lut4_kernel<WIDE, 2, 4><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
@@ -682,14 +684,10 @@ int vq_gemm_mx_rows(const void* a, const void* a_scale, const void* a_levels, in
   p.out = out; p.out_dt = out_dtype;
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.bs = (int)block_size; p.lda = K;
   p.alpha = alpha; p.alpha_dt = alpha_dtype; p.bias = bias; p.bias_dt = bias_dtype;
-  const Lut4Plan q = lut4_plan(M, N, K, true);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  p.counters = static_cast<int*>(workspace);
-  p.workspace = reinterpret_cast<float*>(p.counters + q.tiles);
   // the tiles' counters belong to this call: products of several streams may run at the same time
-  if (cudaMemsetAsync(p.counters, 0, (size_t)q.tiles * sizeof(int), st) != cudaSuccess)
-    return fail(VQ_ECUDA, "vq_gemm_mx_rows: memset");
-  return launch_row_stream<true>(p, st);
+  p.counters = static_cast<int*>(workspace);
+  p.workspace = reinterpret_cast<float*>(p.counters + lut4_plan(M, N, K, true).tiles);
+  return launch_row_stream<true>(p, static_cast<cudaStream_t>(stream));
 }
 
 int vq_pack_lut4(const void* codes, void* packed, int64_t rows, int64_t K, int* bad, void* stream) {
