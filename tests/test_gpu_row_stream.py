@@ -33,3 +33,55 @@ def test_counters_hold_anything_before_a_call():
                                           work.data_ptr(), counters.data_ptr(), torch.cuda.current_stream().cuda_stream),
                          "vq_gemm_lut4")
         assert torch.equal(out, want)
+
+
+def test_captured_call_outlives_a_wider_one():
+    """A graph captured for a narrow weight replays correctly after a much wider weight went through the same entry and
+    after whatever that call freed was handed out again."""
+    import voyager_b200 as vb
+
+    m, k, bs = 3, 2048, 64
+    w = _packed(vb, 1000, k, bs, 3)
+    x = torch.randn(m, k, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda").bfloat16()
+    want = vb.packed.linear_lut4(x, w, out_dtype=torch.float32)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = vb.packed.linear_lut4(x, w, out_dtype=torch.float32)
+    wide = _packed(vb, 128256, 256, bs, 5)
+    vb.packed.linear_lut4(x[:, :256].contiguous(), wide)
+    del wide
+    others = [torch.full((1024 * 4,), 7, dtype=torch.int32, device="cuda") for _ in range(64)]   # 16 KB each
+    for _ in range(3):
+        out.fill_(float("nan"))
+        graph.replay()
+        assert torch.equal(out, want)
+    assert all(bool((t == 7).all()) for t in others)
+
+
+@pytest.mark.parametrize("packed", [True, False])
+def test_two_streams_at_a_time(packed):
+    import voyager_b200 as vb
+
+    m, k, bs = 2, 4096, 64
+    x = torch.randn(m, k, generator=torch.Generator(device="cuda").manual_seed(6), device="cuda").bfloat16()
+    calls = []
+    for seed in (7, 8):
+        w = _packed(vb, 2000, k, bs, seed)
+        if packed:
+            calls.append(lambda w=w: vb.packed.linear_lut4(x, w, out_dtype=torch.float32))
+        else:
+            codes, ones = vb.packed.unpack_lut4_weight(w), torch.ones(m, k // bs, device="cuda").bfloat16()
+            calls.append(lambda w=w, codes=codes, ones=ones: torch.ops.quantized_ops.linear_mx(
+                x, codes, None, input_scale=ones, weight_scale=w.scale, block_size=bs, weight_code=w.levels,
+                out_dtype=torch.float32))
+    want = [call() for call in calls]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in calls]
+    got = [[], []]
+    for _ in range(50):
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                got[i].append(calls[i]())
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert all(torch.equal(g, want[i]) for g in got[i])

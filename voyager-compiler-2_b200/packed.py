@@ -69,19 +69,13 @@ def unpack_lut4_weight(weight: PackedLUT4Weight) -> torch.Tensor:
     return nib.to(torch.bfloat16)
 
 
-_counters = {}
-
-
 def _scratch(device, m, n, k):
-    """Float32 partial-sum workspace for this call and the device's tile counters (zero between calls)."""
+    """This call's partial sums (float32) followed by its tile counters, as one tensor, and where the counters begin.
+    Nothing is kept: a buffer held for the next call would be shared by streams that run at the same time, and
+    replacing it by a larger one would leave a captured graph with an address that is no longer its own."""
     lib = N.lib()
-    work = torch.empty(int(lib.vq_gemm_lut4_workspace_floats(m, n, k)), dtype=torch.float32, device=device)
-    need = int(lib.vq_gemm_lut4_counters(n))
-    have = _counters.get(device)
-    if have is None or have.numel() < need:
-        have = torch.zeros(max(need, 4096), dtype=torch.int32, device=device)
-        _counters[device] = have
-    return work, have
+    floats = int(lib.vq_gemm_lut4_workspace_floats(m, n, k))
+    return torch.empty(floats + int(lib.vq_gemm_lut4_counters(n)), dtype=torch.float32, device=device), floats
 
 
 @N.device_guarded
@@ -119,11 +113,11 @@ def linear_lut4(input: torch.Tensor, weight: PackedLUT4Weight, bias: Optional[to
     if bias is not None:
         bias = bias.contiguous()
     out = torch.empty((m, n), dtype=dtype, device=x.device)
-    work, counters = _scratch(x.device, m, n, k)
+    work, floats = _scratch(x.device, m, n, k)
     N.check(N.lib().vq_gemm_lut4(x.data_ptr(), k, _ptr(scale), _ptr(code), 0 if code is None else code.numel(), m,
                                  weight.codes.data_ptr(), weight.scale.data_ptr(), weight.levels.data_ptr(),
                                  weight.block_size, out.data_ptr(), _dtype_id(dtype), n, k, _ptr(alpha),
                                  0 if alpha is None else _dtype_id(alpha.dtype), _ptr(bias),
-                                 0 if bias is None else _dtype_id(bias.dtype), work.data_ptr(), counters.data_ptr(),
-                                 _stream()), "vq_gemm_lut4")
+                                 0 if bias is None else _dtype_id(bias.dtype), work.data_ptr(),
+                                 work.data_ptr() + 4 * floats, _stream()), "vq_gemm_lut4")
     return out.reshape(*lead, n)
