@@ -665,6 +665,11 @@ int vq_gemm_mx_rows(const void* a, const void* a_scale, const void* a_levels, in
                     int64_t N, int64_t K, const void* alpha, int alpha_dtype, const void* bias, int bias_dtype,
                     void* workspace, void* stream);
 
+/* How those two cut the contraction (host arithmetic only): K is `steps` steps of 128 weights (`packed`: vq_gemm_lut4) or
+ * 32 (vq_gemm_mx_rows) in `slices` slices, of which number `slice` holds steps *begin .. *end - 1. */
+int vq_row_stream_slice(int64_t M, int64_t N, int64_t K, int packed, int64_t slice, int64_t* steps, int64_t* slices,
+                        int64_t* begin, int64_t* end);
+
 /* Packs bfloat16-valued codebook indices codes [rows, K] (each 0..15, what quantize_mx returns
  * for a lookup format with an index table, quantize_pt2e.py:754-791) into vq_gemm_lut4's
  * w_packed layout.  *bad (device int, zeroed by the caller) is set if a value is not such an index. */

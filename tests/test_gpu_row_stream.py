@@ -85,3 +85,25 @@ def test_two_streams_at_a_time(packed):
     torch.cuda.synchronize()
     for i in range(2):
         assert all(torch.equal(g, want[i]) for g in got[i])
+
+
+@pytest.mark.parametrize("m,k", [(2, 327680), (32, 134144)])   # 160 and 150 slices: more than there are SMs
+@pytest.mark.parametrize("packed", [True, False])
+def test_more_slices_than_sms(packed, m, k):
+    import voyager_b200 as vb
+
+    bs, n = 64, 24
+    w = _packed(vb, n, k, bs, 9)
+    x = torch.randn(m, k, generator=torch.Generator(device="cuda").manual_seed(10), device="cuda").bfloat16()
+    codes = vb.packed.unpack_lut4_weight(w)
+    if packed:
+        got = vb.packed.linear_lut4(x, w, out_dtype=torch.float32)
+    else:
+        got = torch.ops.quantized_ops.linear_mx(x, codes, None, input_scale=torch.ones(m, k // bs, device="cuda").bfloat16(),
+                                                weight_scale=w.scale, block_size=bs, weight_code=w.levels,
+                                                out_dtype=torch.float32)
+    vb.ops.gemm_status()
+    real = (w.levels[codes.long()].float() * w.scale.float().repeat_interleave(bs, 1)).bfloat16().double()
+    # float32 sums of k exact products: random-walk rounding of about sqrt(k) 2^-24 of the terms' size
+    bound = 4 * k ** 0.5 * 2.0 ** -24 * (x.double().abs() @ real.abs().T)
+    assert bool(((got.double() - x.double() @ real.T).abs() <= bound).all())

@@ -1,5 +1,8 @@
 """Host side of the weight-streaming linears: workspaces and the cut of the weight."""
 
+import ctypes
+
+import pytest
 import torch
 
 import voyager_b200 as vb
@@ -12,3 +15,27 @@ def test_scratch_belongs_to_one_call():
     for i, one in enumerate(spans):
         for other in spans[:i]:
             assert all(a[1] <= b[0] or b[1] <= a[0] for a in one for b in other)
+
+
+def _slice(rows, n, k, packed, i):
+    values = [ctypes.c_int64() for _ in range(4)]
+    vb._native.check(vb._native.lib().vq_row_stream_slice(rows, n, k, packed, i, *map(ctypes.byref, values)), "slice")
+    return [v.value for v in values]
+
+
+@pytest.mark.parametrize("rows", [1, 9, 17, 25])
+@pytest.mark.parametrize("packed", [0, 1])
+@pytest.mark.parametrize("k", [128, 4096, 14336, 327680, 11_108_352, 16_777_216, 33_554_432, (1 << 30) - 128, (1 << 31) - 128])
+def test_slices_cover_the_contraction(rows, packed, k):
+    n = 4096 if k < 1 << 24 else 16
+    steps, slices, begin, _ = _slice(rows, n, k, packed, 0)
+    assert steps == k // (128 if packed else 32) and 1 <= slices <= steps and begin == 0
+    # the longest slice that the shared memory holds, in steps
+    longest = {(1, 0): 64, (9, 0): 32, (17, 0): 40, (25, 0): 28, (1, 1): 16, (9, 1): 8, (17, 1): 10, (25, 1): 8}[rows, packed]
+    picks = range(slices) if slices < 20000 else sorted({0, 1, slices // 3, slices // 2, slices - 2, slices - 1,
+                                                         *range(0, slices, slices // 500)})
+    for i in picks:
+        _, _, begin, end = _slice(rows, n, k, packed, i)
+        assert begin == i * steps // slices and end == (i + 1) * steps // slices, i
+        assert 1 <= end - begin <= longest
+    assert _slice(rows, n, k, packed, slices - 1)[3] == steps

@@ -117,10 +117,12 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t v, uint32_t s) {
   return r;
 }
 
-// first step of slice `s` (the product is below 2^31: a slice is a few steps long)
-__host__ __device__ inline int l4_slice_begin(int s, int steps, int slices) { return (int)((uint32_t)s * (uint32_t)steps / (uint32_t)slices); }
-// part `i` of `n` equal parts of `total` begins here, and the part that holds step f.  `small`: total * n fits 32 bits
-// (64-bit divisions took half of a tile's finishing).
+// first step of slice `s`.  `small`: steps * slices fits 32 bits (K below 11 million in any plan; 64-bit divisions took
+// half of a tile's finishing)
+__host__ __device__ inline int l4_slice_begin(int s, int steps, int slices, bool small) {
+  return small ? (int)((uint32_t)s * (uint32_t)steps / (uint32_t)slices) : (int)((uint64_t)s * (uint64_t)steps / (uint64_t)slices);
+}
+// part `i` of `n` equal parts of `total` begins here, and the part that holds step f.  `small`: total * n fits 32 bits.
 __device__ inline int l4_cut(uint32_t i, uint32_t total, uint32_t n, bool small) {
   return small ? (int)(i * total / n) : (int)((uint64_t)i * total / n);
 }
@@ -181,9 +183,9 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 
   const int g = lane >> 2, t = lane & 3;
   const int slice = blockIdx.y;
-  const int step0 = l4_slice_begin(slice, p.steps, p.slices);
-  const int steps = l4_slice_begin(slice + 1, p.steps, p.slices) - step0;         // of K, per tile
   const bool small = p.small != 0;
+  const int step0 = l4_slice_begin(slice, p.steps, p.slices, small);
+  const int steps = l4_slice_begin(slice + 1, p.steps, p.slices, small) - step0;  // of K, per tile
   const int total = p.tiles * steps;
   const int cta0 = l4_cut(blockIdx.x, total, p.ctas, small), cta1 = l4_cut(blockIdx.x + 1, total, p.ctas, small);
   const int f0 = cta0 + l4_cut(warp, cta1 - cta0, L4_WARPS, small), f1 = cta0 + l4_cut(warp + 1, cta1 - cta0, L4_WARPS, small);
@@ -409,7 +411,7 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // the parts of this tile, over all slices and CTAs; mine is number `mine`
     int parts = 0, mine = 0;
     for (int s = lane; s < p.slices; s += 32) {
-      const int n = l4_slice_begin(s + 1, p.steps, p.slices) - l4_slice_begin(s, p.steps, p.slices);
+      const int n = l4_slice_begin(s + 1, p.steps, p.slices, small) - l4_slice_begin(s, p.steps, p.slices, small);
       const int first = l4_part_of(tile * n, p.tiles * n, p.ctas, small);
       const int last = l4_part_of((tile + 1) * n - 1, p.tiles * n, p.ctas, small);
       parts += last - first + 1;
@@ -574,6 +576,7 @@ int lut4_status(int reset) {
 // How a product is cut: 8 * NT activation rows, weight tiles of 8 * RG rows, K slices, CTAs per slice.
 struct Lut4Plan {
   int nt, rg, tiles, steps, slices, ctas, max_parts, lda_s;
+  bool small;   // every product of the cut's arithmetic fits 32 bits
 };
 static Lut4Plan lut4_plan(int64_t M, int64_t N, int64_t K, bool wide) {
   const int step = wide ? L4Step<true>::value : L4Step<false>::value;
@@ -601,6 +604,8 @@ static Lut4Plan lut4_plan(int64_t M, int64_t N, int64_t K, bool wide) {
   const int64_t least = total / q.ctas < 1 ? 1 : total / q.ctas;
   const int64_t per_slice = (slice_max - 1) / least + 2;
   q.max_parts = (int)(q.slices * (per_slice < q.ctas ? per_slice : q.ctas));
+  const int64_t most_ctas = q.ctas > L4_WARPS ? q.ctas : L4_WARPS;
+  q.small = ((int64_t)q.tiles * q.steps + 1) * most_ctas < (1ll << 32) && (int64_t)q.steps * q.slices < (1ll << 32);
   return q;
 }
 
@@ -612,8 +617,7 @@ static int launch_row_stream(Lut4Params p, cudaStream_t st) {
   p.tiles = q.tiles; p.steps = q.steps; p.slices = q.slices; p.ctas = q.ctas; p.max_parts = q.max_parts; p.lda_s = q.lda_s;
   while ((1 << p.bs_shift) < p.bs) ++p.bs_shift;
   VQ_REQUIRE(p.slices <= 65535 && (int64_t)q.tiles * q.steps < (1ll << 31), "row stream: weight too large");
-  const int64_t most_ctas = q.ctas > L4_WARPS ? q.ctas : L4_WARPS;
-  p.small = ((int64_t)q.tiles * q.steps + 1) * most_ctas < (1ll << 32);
+  p.small = q.small;
   // Shared memory: the table must sit at shared address L4_TABLE_ADDR.  Dynamic memory starts somewhere in
   // [1 KB, 4 KB) of the window (system + static variables), so reserving up to the table's end measured from
   // 1 KB always suffices; scale slots and partial tiles (16 + 32 KB at most) fit before the table.
@@ -647,6 +651,20 @@ static int launch_row_stream(Lut4Params p, cudaStream_t st) {
 }
 
 extern "C" {
+
+int vq_row_stream_slice(int64_t M, int64_t N, int64_t K, int packed, int64_t slice, int64_t* steps, int64_t* slices,
+                        int64_t* begin, int64_t* end) {
+  VQ_REQUIRE(M > 0 && M <= 32 && N > 0 && N < (1ll << 31) && K > 0 && K < (1ll << 31) && K % (packed ? 128 : 32) == 0,
+             "vq_row_stream_slice: bad extents");
+  VQ_REQUIRE(steps && slices && begin && end, "vq_row_stream_slice: null argument");
+  const Lut4Plan q = lut4_plan(M, N, K, !packed);
+  VQ_REQUIRE(slice >= 0 && slice < q.slices, "vq_row_stream_slice: there are %d slices", q.slices);
+  *steps = q.steps;
+  *slices = q.slices;
+  *begin = l4_slice_begin((int)slice, q.steps, q.slices, q.small);
+  *end = l4_slice_begin((int)slice + 1, q.steps, q.slices, q.small);
+  return VQ_OK;
+}
 
 int64_t vq_gemm_lut4_workspace_floats(int64_t M, int64_t N, int64_t K) {
   if (M <= 0 || N <= 0 || K <= 0 || M > 32 || K % 128) return 0;
