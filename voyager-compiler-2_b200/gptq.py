@@ -65,9 +65,8 @@ def _inverse_factor(h):
     # with rows and columns reversed, the inverse of h's lower factor is the upper factor of the inverse
     k = h.shape[0]
     n = -(-k // 128) * 128
-    work = torch.flip(h, (0, 1)) if n == k else torch.eye(n, dtype=h.dtype, device=h.device)
-    if n != k:
-        work[:k, :k] = torch.flip(h, (0, 1))
+    work = torch.empty(n, n, dtype=h.dtype, device=h.device) if n == k else torch.eye(n, dtype=h.dtype, device=h.device)
+    work[:k, :k] = torch.flip(h, (0, 1))   # a copy into rows of its own: flip() keeps its operand's strides
     panel = torch.empty(n * 128, dtype=torch.float32, device=h.device)
     info = torch.empty((), dtype=torch.int32, device=h.device)
     N.check(N.lib().vq_gptq_factor(work.data_ptr(), panel.data_ptr(), n, info.data_ptr(), _stream()), "vq_gptq_factor")
