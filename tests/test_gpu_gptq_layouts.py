@@ -28,3 +28,13 @@ def test_strides_do_not_matter(k):
     q = vb.get_quantization_map("uint4", "cuda")
     solve = lambda hessian: vb.gptq.compensate_weight_affine(w, hessian, 7, q, 0.0, 15.0, min(k, 128), 0.01)  # noqa: E731
     assert torch.equal(solve(h.T.contiguous().T), solve(h))
+
+
+@pytest.mark.parametrize("k", [5, 128, 200])
+def test_only_the_lower_triangle_is_read(k):
+    import voyager_b200 as vb
+
+    h = _hessian(k)
+    want = vb.gptq.hessian_inverse_chol(h, 7, 0.01)
+    half = h.tril() + torch.full_like(h, 1e6).triu(1)
+    assert torch.equal(vb.gptq.hessian_inverse_chol(half, 7, 0.01), want)

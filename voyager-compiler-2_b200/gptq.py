@@ -66,7 +66,9 @@ def _inverse_factor(h):
     k = h.shape[0]
     n = -(-k // 128) * 128
     work = torch.empty(n, n, dtype=h.dtype, device=h.device) if n == k else torch.eye(n, dtype=h.dtype, device=h.device)
-    work[:k, :k] = torch.flip(h, (0, 1))   # a copy into rows of its own: flip() keeps its operand's strides
+    # a copy into rows of its own: flip() keeps its operand's strides.  The kernel reads the copy's lower triangle, which
+    # is h's when it is h's transpose that is reversed.
+    work[:k, :k] = torch.flip(h.mT, (0, 1))
     panel = torch.empty(n * 128, dtype=torch.float32, device=h.device)
     info = torch.empty((), dtype=torch.int32, device=h.device)
     N.check(N.lib().vq_gptq_factor(work.data_ptr(), panel.data_ptr(), n, info.data_ptr(), _stream()), "vq_gptq_factor")
