@@ -123,6 +123,7 @@ struct TrainCastParams {
   __nv_bfloat16 *t, *t_t;
   int64_t M, K;
   bool wide;             // the input is 32-byte aligned
+  unsigned col_tiles;    // blockIdx.x counts the tiles row by row (a grid's second extent would end at 4 million rows)
 };
 
 struct __align__(16) TrainTile {
@@ -179,13 +180,13 @@ template <bool ROTATE, bool SEED, bool SEED_T>
 __global__ void __launch_bounds__(256, 3)
 cast_pair_kernel(const __grid_constant__ TrainCastParams P) {
   __shared__ TrainTile s;
-  const int64_t k0 = (int64_t)blockIdx.x * kTileK, m0 = (int64_t)blockIdx.y * kTileM;
+  const int64_t k0 = (int64_t)(blockIdx.x % P.col_tiles) * kTileK, m0 = (int64_t)(blockIdx.x / P.col_tiles) * kTileM;
   if (ROTATE) stage_matrix(s.m, P.matrix);
   Words8 x[2];
   load_tile(P, s, m0, k0, x);
   const GlobalScale g = nv_make_global(nv_global_scale(P.amax[0]));
   const GlobalScale gt = ROTATE ? nv_make_global(nv_global_scale(P.amax[1])) : g;
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     *P.t = __float2bfloat16_rn(g.t);
     *P.t_t = __float2bfloat16_rn(gt.t);
   }
@@ -227,12 +228,12 @@ cast_square_kernel(const __grid_constant__ TrainCastParams P) {
   __shared__ uint16_t row_max[kTileM][8];
   __shared__ float block_es[4][8];
   __shared__ uint32_t block_sb[4][8];
-  const int64_t k0 = (int64_t)blockIdx.x * kTileK, m0 = (int64_t)blockIdx.y * kTileM;
+  const int64_t k0 = (int64_t)(blockIdx.x % P.col_tiles) * kTileK, m0 = (int64_t)(blockIdx.x / P.col_tiles) * kTileM;
   const int row = threadIdx.x >> 2;
   Words8 x[2];
   load_tile(P, s, m0, k0, x);
   const GlobalScale g = nv_make_global(nv_global_scale(P.amax[0]));
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *P.t = __float2bfloat16_rn(g.t);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *P.t = __float2bfloat16_rn(g.t);
 #pragma unroll
   for (int b = 0; b < 2; ++b)
     if (k0 + b * 64 < P.K) row_max[row][b * 4 + (threadIdx.x & 3)] = (uint16_t)nv_amax16(x[b].w);
@@ -277,9 +278,11 @@ int zero_ragged_scales(void* scales, int64_t rows, int64_t K, cudaStream_t st) {
   return VQ_OK;
 }
 
+int64_t tile_count(const TrainCastParams& P) { return P.M / kTileM * P.col_tiles; }
+
 int check_train_cast(const TrainCastParams& P, const char* what) {
   VQ_REQUIRE(P.M > 0 && P.K > 0 && P.M % 64 == 0 && P.K % 64 == 0, "%s: both extents must be positive multiples of 64", what);
-  VQ_REQUIRE(P.M / kTileM <= 65535 && P.K < (1ll << 31), "%s: matrix too large", what);
+  VQ_REQUIRE(P.K < (1ll << 31) && tile_count(P) < (1ll << 31), "%s: matrix too large", what);
   VQ_REQUIRE(P.in && P.amax && P.codes && P.scales && P.codes_t && P.scales_t && P.t, "%s: null argument", what);
   VQ_REQUIRE(((reinterpret_cast<uintptr_t>(P.in) | reinterpret_cast<uintptr_t>(P.codes) | reinterpret_cast<uintptr_t>(P.scales) |
                reinterpret_cast<uintptr_t>(P.codes_t) | reinterpret_cast<uintptr_t>(P.scales_t)) & 15) == 0 &&
@@ -298,7 +301,7 @@ extern "C" int vq_cast_nvfp4_pair(const void* in, const float* matrix, const int
   TrainCastParams P{static_cast<const char*>(in), matrix, amax, seed, seed_t, static_cast<uint8_t*>(codes),
                     static_cast<uint8_t*>(scales), static_cast<uint8_t*>(codes_t), static_cast<uint8_t*>(scales_t),
                     static_cast<__nv_bfloat16*>(t), static_cast<__nv_bfloat16*>(t_t), M, K,
-                    (reinterpret_cast<uintptr_t>(in) & 31) == 0};
+                    (reinterpret_cast<uintptr_t>(in) & 31) == 0, (unsigned)((K + kTileK - 1) / kTileK)};
   if (int e = check_train_cast(P, "vq_cast_nvfp4_pair")) return e;
   VQ_REQUIRE(t_t, "vq_cast_nvfp4_pair: null argument");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -314,7 +317,7 @@ extern "C" int vq_cast_nvfp4_pair(const void* in, const float* matrix, const int
   } else if (int e = vq_amax(in, VQ_BF16, M * K, amax, stream)) {
     return e;
   }
-  const dim3 grid((unsigned)((K + kTileK - 1) / kTileK), (unsigned)(M / kTileM));
+  const unsigned grid = (unsigned)tile_count(P);
 #define VQ_PAIR(R) \
   (seed ? (seed_t ? cast_pair_kernel<R, true, true><<<grid, 256, 0, st>>>(P) : cast_pair_kernel<R, true, false><<<grid, 256, 0, st>>>(P)) \
         : (seed_t ? cast_pair_kernel<R, false, true><<<grid, 256, 0, st>>>(P) : cast_pair_kernel<R, false, false><<<grid, 256, 0, st>>>(P)))
@@ -329,13 +332,13 @@ extern "C" int vq_cast_nvfp4_square(const void* in, float* amax, void* codes, vo
   TrainCastParams P{static_cast<const char*>(in), nullptr, amax, nullptr, nullptr, static_cast<uint8_t*>(codes),
                     static_cast<uint8_t*>(scales), static_cast<uint8_t*>(codes_t), static_cast<uint8_t*>(scales_t),
                     static_cast<__nv_bfloat16*>(t), nullptr, N, K,
-                    (reinterpret_cast<uintptr_t>(in) & 31) == 0};
+                    (reinterpret_cast<uintptr_t>(in) & 31) == 0, (unsigned)((K + kTileK - 1) / kTileK)};
   if (int e = check_train_cast(P, "vq_cast_nvfp4_square")) return e;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(amax, 0, sizeof(float), st) != cudaSuccess) return fail(VQ_ECUDA, "vq_cast_nvfp4_square: memset");
   if (int e = zero_ragged_scales(scales, N, K, st)) return e;
   if (int e = zero_ragged_scales(scales_t, K, N, st)) return e;
   if (int e = vq_amax(in, VQ_BF16, N * K, amax, stream)) return e;
-  cast_square_kernel<<<dim3((unsigned)((K + kTileK - 1) / kTileK), (unsigned)(N / kTileM)), 256, 0, st>>>(P);
+  cast_square_kernel<<<(unsigned)tile_count(P), 256, 0, st>>>(P);
   return check_launch("cast_square_kernel");
 }
