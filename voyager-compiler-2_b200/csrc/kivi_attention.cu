@@ -469,10 +469,14 @@ extern "C" int vq_kivi_decode_attention(const void* q, const void* k_packed, con
                 "vq_kivi_decode_attention: needs head_dim 128, at most 8 query heads per KV head, key groups of a "
                 "multiple of 64 positions, value groups of 32, 64 or 128 channels, 16 recent positions or more (or "
                 "none) and the scores of a CTA's share of the positions beside two staged chunks within 227 KB of shared memory");
-  VQ_REQUIRE(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_packed) | reinterpret_cast<uintptr_t>(k_scale) |
-               reinterpret_cast<uintptr_t>(k_zero) | reinterpret_cast<uintptr_t>(v_packed) | reinterpret_cast<uintptr_t>(v_scale) |
-               reinterpret_cast<uintptr_t>(v_zero) | reinterpret_cast<uintptr_t>(k_res) | reinterpret_cast<uintptr_t>(v_res)) & 15) == 0,
-             "vq_kivi_decode_attention: buffers must be 16-byte aligned");
+  const uintptr_t addresses =
+      reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_packed) | reinterpret_cast<uintptr_t>(k_scale) |
+      reinterpret_cast<uintptr_t>(k_zero) | reinterpret_cast<uintptr_t>(v_packed) | reinterpret_cast<uintptr_t>(v_scale) |
+      reinterpret_cast<uintptr_t>(v_zero) | reinterpret_cast<uintptr_t>(k_res) | reinterpret_cast<uintptr_t>(v_res);
+  // a window of any length may be a slice that begins anywhere: the caller's operators take it
+  if (R % 16 != 0 && (addresses & 15) != 0)
+    return fail(VQ_EUNSUPPORTED, "vq_kivi_decode_attention: a window that is no multiple of 16 positions needs 16-byte aligned buffers");
+  VQ_REQUIRE((addresses & 15) == 0, "vq_kivi_decode_attention: buffers must be 16-byte aligned");
   KaParams p;
   p.q = static_cast<const __nv_bfloat16*>(q);
   p.k_packed = static_cast<const uint8_t*>(k_packed);
