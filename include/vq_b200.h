@@ -658,7 +658,8 @@ int vq_gemm_lut4(const void* a, int64_t lda, const void* a_scale, const void* a_
 /* linear_mx (ops/quantized.py:662-723) for at most 32 activation rows on the operator's own storage: a [M, K] and w
  * [N, K] bfloat16 codes with bfloat16 scales per `block_size` elements of K ([M, K / bs], [N, K / bs]); a_levels / w_levels:
  * bfloat16 codebooks (w_levels 16 entries) or null when the codes are the values.  K is a multiple of 32 and of the
- * block size (a power of two, 8 or more).  workspace: vq_gemm_mx_rows_workspace_bytes(M, N, K) bytes. */
+ * block size (a power of two, 8 or more).  workspace: vq_gemm_mx_rows_workspace_bytes(M, N, K) bytes; 0 where the kernel does
+ * not take the extents (more than 65535 K slices: K above 58 million or more, depending on M). */
 int64_t vq_gemm_mx_rows_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int vq_gemm_mx_rows(const void* a, const void* a_scale, const void* a_levels, int n_a_levels, const void* w,
                     const void* w_scale, const void* w_levels, int64_t block_size, void* out, int out_dtype, int64_t M,

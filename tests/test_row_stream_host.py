@@ -39,3 +39,16 @@ def test_slices_cover_the_contraction(rows, packed, k):
         assert begin == i * steps // slices and end == (i + 1) * steps // slices, i
         assert 1 <= end - begin <= longest
     assert _slice(rows, n, k, packed, slices - 1)[3] == steps
+
+
+@pytest.mark.parametrize("rows,k", [(32, 58_720_256 + 1024), (8, 134_217_728 + 2048), (1, (1 << 30) - 64)])
+def test_too_many_slices_are_left_to_the_gemm(rows, k):
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    assert vb._native.lib().vq_gemm_mx_rows_workspace_bytes(rows, 16, k) == 0
+    assert vb._native.lib().vq_gemm_mx_rows_workspace_bytes(rows, 16, 4096) > 0
+    with FakeTensorMode():
+        codes = lambda r: torch.empty(r, k, dtype=torch.bfloat16, device="cuda")  # noqa: E731
+        scale = lambda r: torch.empty(r, k // 64, dtype=torch.bfloat16, device="cuda")  # noqa: E731
+        assert vb.ops._mx_gemm_few_rows(vb.ops.LINEAR_LAYOUT, codes(rows), codes(16), None, scale(rows), scale(16), 64, None,
+                                        None, None, vb.ops.LINEAR_LAYOUT, torch.float32) is None

@@ -609,6 +609,9 @@ static Lut4Plan lut4_plan(int64_t M, int64_t N, int64_t K, bool wide) {
   return q;
 }
 
+// Slices lie along the grid's second extent, a slice's steps are counted in an int.
+static bool lut4_launchable(const Lut4Plan& q) { return q.slices <= 65535 && (int64_t)q.tiles * q.steps < (1ll << 31); }
+
 // The cut, tensor maps and launch of a product whose operands stand in `p`.
 template <bool WIDE>
 static int launch_row_stream(Lut4Params p, cudaStream_t st) {
@@ -616,7 +619,7 @@ static int launch_row_stream(Lut4Params p, cudaStream_t st) {
   const Lut4Plan q = lut4_plan(M, N, K, WIDE);
   p.tiles = q.tiles; p.steps = q.steps; p.slices = q.slices; p.ctas = q.ctas; p.max_parts = q.max_parts; p.lda_s = q.lda_s;
   while ((1 << p.bs_shift) < p.bs) ++p.bs_shift;
-  VQ_REQUIRE(p.slices <= 65535 && (int64_t)q.tiles * q.steps < (1ll << 31), "row stream: weight too large");
+  VQ_REQUIRE(lut4_launchable(q), "row stream: weight too large");
   p.small = q.small;
   // Shared memory: the table must sit at shared address L4_TABLE_ADDR.  Dynamic memory starts somewhere in
   // [1 KB, 4 KB) of the window (system + static variables), so reserving up to the table's end measured from
@@ -677,6 +680,7 @@ int64_t vq_gemm_lut4_counters(int64_t N) { return N <= 0 ? 0 : (N + 15) / 16; }
 int64_t vq_gemm_mx_rows_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   if (M <= 0 || N <= 0 || K <= 0 || M > 32 || K % 32) return 0;
   const Lut4Plan q = lut4_plan(M, N, K, true);
+  if (!lut4_launchable(q)) return 0;
   return ((int64_t)q.tiles * q.max_parts * (q.nt * 8) * (q.rg * 8) + q.tiles) * 4;
 }
 

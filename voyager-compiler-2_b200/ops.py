@@ -845,14 +845,17 @@ def _mx_gemm_few_rows(native, a, b, bias, input_scale, weight_scale, block_size,
     if not (_scales_per_row(a, input_scale, block_size) and _scales_per_row(b, weight_scale, block_size)
             and _level_table(input_code, 0) and _level_table(weight_code, 16)):
         return None
+    lib = N.lib()
+    scratch = lib.vq_gemm_mx_rows_workspace_bytes(rows, n, k)
+    if scratch == 0:   # a contraction of too many slices
+        return None
     a2, b2 = a.reshape(rows, k).contiguous(), b.contiguous()
     if a2.data_ptr() % 16 or b2.data_ptr() % 16:
         return None
     if bias is not None:
         bias = bias.contiguous()
-    lib = N.lib()
     out = torch.empty((rows, n), dtype=dtype, device=a.device)
-    work = torch.empty(lib.vq_gemm_mx_rows_workspace_bytes(rows, n, k), dtype=torch.uint8, device=a.device)
+    work = torch.empty(scratch, dtype=torch.uint8, device=a.device)
     N.check(lib.vq_gemm_mx_rows(a2.data_ptr(), input_scale.data_ptr(), _ptr(input_code),
                                 0 if input_code is None else input_code.numel(), b2.data_ptr(), weight_scale.data_ptr(),
                                 _ptr(weight_code), block_size, out.data_ptr(), _dtype_id(dtype), rows, n, k, _ptr(alpha),
