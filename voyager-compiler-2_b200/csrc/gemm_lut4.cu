@@ -151,6 +151,15 @@ __device__ __noinline__ uint4 decode_odd(uint4 raw, const __nv_bfloat16* __restr
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
+// Clears the tiles' counters before the product that counts in them.  A kernel, with the product launched as its
+// programmatic dependent (that launch and the product's prologue overlap this one): the decode step of one sequence, four
+// products, takes 133 us in a graph, 146 with a memset node before each and 127 with counters that nothing clears.
+__global__ void __launch_bounds__(256) clear_counters_kernel(int* counters, int n) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < n) counters[i] = 0;
+}
+
 // NT: activation rows in tiles of 8 (1..4).  RG: row groups of 8 per weight tile (4, or 2 beside many activation rows).
 template <bool WIDE, int NT, int RG>
 __global__ void __launch_bounds__(L4_THREADS, 1)
@@ -202,7 +211,7 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   int ft = f0 / steps, fk = f0 - ft * steps;               // next step to fetch
   int to_fetch = f1 - f0, fetch_slot = 1, fetched_piece = -1;
   struct Scales { uint32_t s[RG]; };
-  auto fetch = [&](int stage, Scales& sc) {
+  auto fetch = [&](int stage, Scales& sc, bool early) {
     if (to_fetch <= 0) return;
     --to_fetch;
     if (p.tma_scales) {
@@ -221,20 +230,24 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         tma_load_3d(ring + stage * (TILE * 64), &map_w, &bars[warp][stage], (step0 + fk) * 64, ft * TILE, 0);
       }
 #pragma unroll
-      for (int j = 0; j < RG; ++j)   // rows past the end of the weight read row N - 1's scales; their results are never stored
-        sc.s[j] = __ldg(static_cast<const uint16_t*>(p.w_scale) + (int64_t)min(ft * TILE + 8 * j + g, p.N - 1) * blocks_per_row +
-                        (((step0 + fk) * L4_STEP + t * (L4_STEP / 4)) >> p.bs_shift));
+      for (int j = 0; j < RG; ++j) {   // rows past the end of the weight read row N - 1's scales; their results are never stored
+        const uint16_t* src = static_cast<const uint16_t*>(p.w_scale) + (int64_t)min(ft * TILE + 8 * j + g, p.N - 1) * blocks_per_row +
+                              (((step0 + fk) * L4_STEP + t * (L4_STEP / 4)) >> p.bs_shift);
+        sc.s[j] = early ? __ldcg(src) : __ldg(src);
+      }
     }
     if (++fk == steps) { fk = 0; ++ft; }
   };
   Scales sc0, sc1;
-  fetch(0, sc0);
-  fetch(1, sc1);
+  fetch(0, sc0, true);
+  fetch(1, sc1, true);
 
   // ---- prologue: byte table and the decoded activation slice ----
-  if (threadIdx.x < 16 && p.w_levels) w_levels[threadIdx.x] = static_cast<const uint16_t*>(p.w_levels)[threadIdx.x];
+  // It runs beside the clearing of the counters.  That kernel began after everything before it in the stream had ended, so
+  // the operands are in the L2; loads go there (TMA, ld.cg), not to an L1 that an earlier kernel may have filled.
+  if (threadIdx.x < 16 && p.w_levels) w_levels[threadIdx.x] = __ldcg(static_cast<const uint16_t*>(p.w_levels) + threadIdx.x);
   if (p.a_levels != nullptr && (int)threadIdx.x < p.n_a_levels)
-    a_levels[threadIdx.x] = __bfloat162float(static_cast<const __nv_bfloat16*>(p.a_levels)[threadIdx.x]);
+    a_levels[threadIdx.x] = __uint_as_float((uint32_t)__ldcg(static_cast<const uint16_t*>(p.a_levels) + threadIdx.x) << 16);
   __syncthreads();
   for (int i = threadIdx.x; i < 256 * 32 && p.w_levels; i += L4_THREADS) {
     const int byte = i >> 5;
@@ -242,7 +255,7 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   }
   {
     const __nv_bfloat16* A = static_cast<const __nv_bfloat16*>(p.a);
-    const __nv_bfloat16* S = static_cast<const __nv_bfloat16*>(p.a_scale);
+    const uint16_t* S = static_cast<const uint16_t*>(p.a_scale);
     const bool coded = p.a_levels != nullptr;
     const int k0 = step0 * L4_STEP;
     const int groups = steps * (L4_STEP / 8);                                      // 8 elements per thread and step
@@ -257,8 +270,8 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         raw[u] = make_uint4(0, 0, 0, 0);
         scl[u] = 1.0f;
         if (idx < NT * 8 * groups && m < p.M) {
-          raw[u] = *reinterpret_cast<const uint4*>(A + (int64_t)m * p.lda + k0 + kk);
-          if (S) scl[u] = __bfloat162float(S[(int64_t)m * blocks_per_row + ((k0 + kk) >> p.bs_shift)]);
+          raw[u] = __ldcg(reinterpret_cast<const uint4*>(A + (int64_t)m * p.lda + k0 + kk));
+          if (S) scl[u] = __uint_as_float((uint32_t)__ldcg(S + (int64_t)m * blocks_per_row + ((k0 + kk) >> p.bs_shift)) << 16);
         }
       }
 #pragma unroll
@@ -298,6 +311,7 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       }
     }
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // the counters are clear; nothing was written to global memory before
   __syncthreads();
 
   // This lane's column of the table as a 32-bit shared address; its second byte is zero.
@@ -465,7 +479,7 @@ gemm_lut4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       for (int j = 0; j < RG; ++j) sc[j] = next.s[j] * 0x10001u;
     }
     __syncwarp();   // the step is in registers: its slot may be refilled
-    fetch(stage, next);
+    fetch(stage, next, false);
     if constexpr (WIDE) compute_wide(ck, w8, sc);
     else compute(ck, w8, sc);
     --left;
@@ -643,13 +657,23 @@ static int launch_row_stream(Lut4Params p, cudaStream_t st) {
     cudaFuncSetAttribute(gemm_lut4_kernel<WIDE, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
   }
   // cleared by every call and not by the last launch's tiles: a launch that gave up leaves some of them counted in part
-  if (cudaMemsetAsync(p.counters, 0, (size_t)q.tiles * sizeof(int), st) != cudaSuccess)
-    return fail(VQ_ECUDA, "row stream: memset");
-  const dim3 grid((unsigned)q.ctas, (unsigned)q.slices);
-  if (q.nt == 1) gemm_lut4_kernel<WIDE, 1, 4><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
-  else if (q.nt == 2) gemm_lut4_kernel<WIDE, 2, 4><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
-  else if (q.nt == 3) gemm_lut4_kernel<WIDE, 3, 2><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
-  else gemm_lut4_kernel<WIDE, 4, 2><<<grid, L4_THREADS, smem, st>>>(map_w, map_s, p);
+  clear_counters_kernel<<<(unsigned)((q.tiles + 255) / 256), 256, 0, st>>>(p.counters, q.tiles);
+  if (int e = check_launch("clear_counters_kernel")) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)q.ctas, (unsigned)q.slices);
+  cfg.blockDim = dim3(L4_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = q.nt == 1   ? cudaLaunchKernelEx(&cfg, gemm_lut4_kernel<WIDE, 1, 4>, map_w, map_s, p)
+                        : q.nt == 2 ? cudaLaunchKernelEx(&cfg, gemm_lut4_kernel<WIDE, 2, 4>, map_w, map_s, p)
+                        : q.nt == 3 ? cudaLaunchKernelEx(&cfg, gemm_lut4_kernel<WIDE, 3, 2>, map_w, map_s, p)
+                                    : cudaLaunchKernelEx(&cfg, gemm_lut4_kernel<WIDE, 4, 2>, map_w, map_s, p);
+  if (e != cudaSuccess) return fail(VQ_ECUDA, "gemm_lut4_kernel: %s", cudaGetErrorString(e));
   return check_launch("gemm_lut4_kernel");
 }
 
