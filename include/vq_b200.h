@@ -218,7 +218,11 @@ int vq_hadamard_rotate(const void* in, void* out, int dtype, const float* matrix
 /* hessian_inverse_chol's factorisation (quantization/gptq.py:37-75) in one elimination: W holds the damped Hessian with rows
  * and columns in reverse order, [n, n] float32, n a multiple of 128 (pad with an identity block at the end); on return its
  * lower triangle is L^-1 where W = L L^T, whose reverse in rows and columns is the upper Cholesky factor of the
- * Hessian's inverse.  panel: n * 128 floats of workspace; *info (device) becomes 1 if a pivot was not positive. */
+ * Hessian's inverse.  panel: n * 128 floats of workspace; *info (device) becomes 1 if a pivot was not positive.
+ * vq_gptq_factor_load makes that W [n, n] from the lower triangle of a Hessian h [k, k] whose element (i, j) lies at
+ * i * row_stride + j * col_stride; W's upper triangle becomes zero and stays it. */
+int vq_gptq_factor_load(const float* h, int64_t row_stride, int64_t col_stride, float* W, int64_t k, int64_t n,
+                        void* stream);
 int vq_gptq_factor(float* W, float* panel, int64_t n, int* info, void* stream);
 
 /* One block of the GPTQ column sweep -- quantization/gptq.py: block_scale (85-143)

@@ -137,6 +137,7 @@ SIGNATURES = {
     "vq_gemm_mx_rows_workspace_bytes": [_I64, _I64, _I64],
     "vq_gemm_mx_rows": [_P, _P, _P, _I, _P, _P, _P, _I64, _P, _I, _I64, _I64, _I64, _P, _I, _P, _I, _P, _P],
     "vq_row_stream_slice": [_I64, _I64, _I64, _I, _I64, *[ctypes.POINTER(_I64)] * 4],
+    "vq_gptq_factor_load": [_P, _I64, _I64, _P, _I64, _I64, _P],
     "vq_gptq_factor": [_P, _P, _I64, _P, _P],
     "vq_attention_fp8_ragged": [_P, _P, _P, _I64, _P, _I64, _P, _I64, _I64, _I64, _I64, _P, _I, _F, _P, _I, _P, _I, _P, _I,
                                 _I, _P],

@@ -15,6 +15,28 @@
 namespace vq {
 namespace {
 
+// W = J h^T J from the lower triangle of h (element (i, j) at i * rs + j * cs), zeros above the diagonal, an identity
+// behind row k.  Tiles of 32 x 32 turned in shared memory, so that reads run along h's denser axis and writes along W's
+// rows.  K = 4096: 40 us; reversing the transpose, copying it into rows and masking took 161 as tensor operators.
+__global__ void __launch_bounds__(256)
+factor_load_kernel(const float* __restrict__ h, int64_t rs, int64_t cs, float* __restrict__ W, int64_t k, int64_t n) {
+  __shared__ float s[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t a0 = (int64_t)blockIdx.y * 32, b0 = (int64_t)blockIdx.x * 32;
+  const bool along_rows = cs <= rs;
+#pragma unroll
+  for (int u = 0; u < 32; u += 8) {
+    const int al = along_rows ? tx : ty + u, bl = along_rows ? ty + u : tx;
+    const int64_t a = a0 + al, b = b0 + bl;
+    float v = a == b ? 1.0f : 0.0f;
+    if (a < k && b < k) v = b <= a ? __ldg(h + (k - 1 - b) * rs + (k - 1 - a) * cs) : 0.0f;
+    s[al][bl] = v;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 32; u += 8) W[(a0 + ty + u) * n + b0 + tx] = s[ty + u][tx];
+}
+
 // One 128 x 128 block: 512 threads own 4 x 8 elements each in registers, a warp 16 x 64.  Column c's raw values and row
 // c's go through shared memory (two buffers, one barrier per column); then every thread eliminates its own elements: a
 // factor of zero leaves the finished rows alone.  Warps whose rows are all finished, or lie above the diagonal, only
@@ -139,6 +161,17 @@ factor_update_kernel(float* __restrict__ W, const float* __restrict__ P, int64_t
 }  // namespace vq
 
 using namespace vq;
+
+extern "C" int vq_gptq_factor_load(const float* h, int64_t row_stride, int64_t col_stride, float* W, int64_t k, int64_t n,
+                                   void* stream) {
+  VQ_REQUIRE(k >= 0 && n >= k && n % 128 == 0 && n <= (1 << 20) && row_stride >= 0 && col_stride >= 0,
+             "vq_gptq_factor_load: bad extents");
+  if (n == 0) return VQ_OK;
+  VQ_REQUIRE(W && (h || k == 0), "vq_gptq_factor_load: null argument");
+  const unsigned tiles = (unsigned)(n / 32);
+  factor_load_kernel<<<dim3(tiles, tiles), 256, 0, static_cast<cudaStream_t>(stream)>>>(h, row_stride, col_stride, W, k, n);
+  return check_launch("factor_load_kernel");
+}
 
 extern "C" int vq_gptq_factor(float* W, float* panel, int64_t n, int* info, void* stream) {
   VQ_REQUIRE(n >= 0 && n % 128 == 0 && n <= (1 << 20), "vq_gptq_factor: the extent must be a multiple of 128");

@@ -65,14 +65,13 @@ def _inverse_factor(h):
     # with rows and columns reversed, the inverse of h's lower factor is the upper factor of the inverse
     k = h.shape[0]
     n = -(-k // 128) * 128
-    work = torch.empty(n, n, dtype=h.dtype, device=h.device) if n == k else torch.eye(n, dtype=h.dtype, device=h.device)
-    # a copy into rows of its own: flip() keeps its operand's strides.  The kernel reads the copy's lower triangle, which
-    # is h's when it is h's transpose that is reversed.
-    work[:k, :k] = torch.flip(h.mT, (0, 1))
+    work = torch.empty(n, n, dtype=h.dtype, device=h.device)
+    N.check(N.lib().vq_gptq_factor_load(h.data_ptr(), h.stride(0), h.stride(1), work.data_ptr(), k, n, _stream()),
+            "vq_gptq_factor_load")
     panel = torch.empty(n * 128, dtype=torch.float32, device=h.device)
     info = torch.empty((), dtype=torch.int32, device=h.device)
     N.check(N.lib().vq_gptq_factor(work.data_ptr(), panel.data_ptr(), n, info.data_ptr(), _stream()), "vq_gptq_factor")
-    return torch.flip(work.tril_()[:k, :k], (0, 1)), info
+    return torch.flip(work[:k, :k], (0, 1)), info
 
 
 def salience_order(hessian, columns, within_block, block_size):
