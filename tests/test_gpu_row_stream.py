@@ -87,7 +87,7 @@ def test_two_streams_at_a_time(packed):
         assert all(torch.equal(g, want[i]) for g in got[i])
 
 
-@pytest.mark.parametrize("m,k", [(2, 327680), (32, 134144)])   # 160 and 150 slices: more than there are SMs
+@pytest.mark.parametrize("m,k", [(2, 327680), (32, 153600)])   # 150 slices and more: there are 148 SMs
 @pytest.mark.parametrize("packed", [True, False])
 def test_more_slices_than_sms(packed, m, k):
     import voyager_b200 as vb
@@ -107,3 +107,47 @@ def test_more_slices_than_sms(packed, m, k):
     # float32 sums of k exact products: random-walk rounding of about sqrt(k) 2^-24 of the terms' size
     bound = 4 * k ** 0.5 * 2.0 ** -24 * (x.double().abs() @ real.abs().T)
     assert bool(((got.double() - x.double() @ real.T).abs() <= bound).all())
+
+
+def _off(t):
+    """The same values two bytes past a 16-byte boundary."""
+    flat = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+    at = flat[1:t.numel() + 1]
+    at.copy_(t.reshape(-1))
+    assert at.data_ptr() % 16 == 2
+    return at.view(t.shape)
+
+
+@pytest.mark.parametrize("m", [3, 20])
+@pytest.mark.parametrize("n,k,bs", [(40, 4096, 64), (33, 1024, 16)])
+@pytest.mark.parametrize("coded", [False, True])
+@pytest.mark.parametrize("off", [False, True])
+def test_special_scales_and_scales_anywhere(m, n, k, bs, coded, off):
+    """Infinite and NaN scales, zero ones beside infinite ones, and scale rows that TMA cannot fetch: the streamed product
+    has the read-back path's infinities and NaNs, and its values up to the order of the sums."""
+    import voyager_b200 as vb
+
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a, w = (torch.randint(0, 16, (r, k), generator=g, device="cuda").bfloat16() for r in (m, n))
+    sa, sw = ((torch.rand(r, k // bs, generator=g, device="cuda") + 0.5).bfloat16() for r in (m, n))
+    a[1], w[1] = 3.0, 9.0       # products of one sign: an infinite scale gives an infinity and not their difference
+    sw[1, 2], sw[n - 1, 0], sw[5, 3], sa[2, 1], sa[0, 3] = float("inf"), float("nan"), -float("inf"), float("inf"), 0.0
+    levels = torch.linspace(-1, 1, 16, device="cuda").bfloat16() if coded else None
+    if off:
+        sa, sw = _off(sa), _off(sw)
+    layout = vb.ops.LINEAR_LAYOUT
+    got = vb.ops._mx_gemm_few_rows(layout, a, w, None, sa, sw, bs, levels, levels, None, layout, torch.float32)
+    assert got is not None
+    real_a, real_w = (torch.ops.quantized_ops.dequantize_mx(c, s, bs, levels) for c, s in ((a, sa), (w, sw)))
+    want = real_a.double() @ real_w.double().T
+    assert torch.equal(got.isnan(), want.isnan()) and bool(want.isnan().any()) and bool(want.isinf().any())
+    assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[want.isinf()], want[want.isinf()].float())
+    # float32 sums of k exact products: random-walk rounding of about sqrt(k) 2^-24 of the terms' size
+    bound = 4 * k ** 0.5 * 2.0 ** -24 * (real_a.double().abs() @ real_w.double().abs().T)
+    finite = want.isfinite()
+    assert bool(((got.double() - want).abs() <= bound)[finite].all())
+    if coded and bs >= 32:
+        packed = vb.packed.PackedLUT4Weight(vb.packed.pack_lut4_weight(w, sw, levels, bs).codes, sw, levels, bs)
+        again = vb.packed.linear_lut4(a, packed, input_scale=sa, input_code=levels, out_dtype=torch.float32)
+        assert torch.equal(again.isnan(), want.isnan()) and torch.equal(again.isinf(), want.isinf())
+        assert bool(((again.double() - want).abs() <= bound)[finite].all())
