@@ -1050,8 +1050,8 @@ class C5:
     description = ("c5: GPTQ 4-bit asymmetric group-wise quantization (group 128, damp 0.01, act-order off) of ONE "
                    "Llama-3.1-8B-shaped decoder layer's 7 linears per step (the model is 32 such layers, 224 linears), "
                    "calibration 128 x 2048 = 262144 tokens per linear, N(0,1) mixed with a rank-64 component: per linear "
-                   "the Hessian X^T X on the tensor cores streamed in 16384-row chunks, damped Cholesky inverse "
-                   "(torch.linalg on the device), blocked column sweep + trailing updates (CUDA kernels). tok/s = "
+                   "the Hessian X^T X on the tensor cores streamed in 16384-row chunks, damped inverse's Cholesky "
+                   "factor in one elimination, blocked column sweep + trailing updates (CUDA kernels). tok/s = "
                    "calibration tokens / (32 x the layer's time)")
     tokens = calibration // 32
     n_sets = 1
