@@ -52,3 +52,26 @@ def test_too_many_slices_are_left_to_the_gemm(rows, k):
         scale = lambda r: torch.empty(r, k // 64, dtype=torch.bfloat16, device="cuda")  # noqa: E731
         assert vb.ops._mx_gemm_few_rows(vb.ops.LINEAR_LAYOUT, codes(rows), codes(16), None, scale(rows), scale(16), 64, None,
                                         None, None, vb.ops.LINEAR_LAYOUT, torch.float32) is None
+
+
+def _route(rows, n, k, bs, lookup):
+    """What linear_mx's few-rows path makes of a call: None where it leaves it to the GEMM."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    with FakeTensorMode():
+        make = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device="cuda")  # noqa: E731
+        levels = make(16) if lookup else None
+        try:
+            return vb.ops._mx_gemm_few_rows(vb.ops.LINEAR_LAYOUT, make(rows, k), make(n, k), None, make(rows, k // bs),
+                                            make(n, k // bs), bs, levels, levels, None, vb.ops.LINEAR_LAYOUT, torch.bfloat16)
+        except RuntimeError:   # it went on to the kernel, which takes no tensor without memory
+            return "streamed"
+
+
+@pytest.mark.parametrize("rows,n,k,lookup,streamed", [
+    (1, 128256, 4096, True, True), (24, 128256, 4096, True, True), (24, 18944, 4096, False, True), (24, 512, 128, False, True),
+    (25, 8448, 4096, True, True), (32, 10240, 5120, True, True), (32, 14336, 4096, True, False), (25, 22016, 4096, True, False),
+    (32, 12288, 10752, True, True), (32, 14336, 4096, False, True), (32, 18944, 4096, False, False),
+    (32, 22016, 4096, False, True), (25, 37888, 4096, False, False), (32, 128256, 4096, False, False), (33, 512, 512, False, False)])
+def test_which_products_are_streamed(rows, n, k, lookup, streamed):
+    assert (_route(rows, n, k, 64, lookup) is not None) == streamed

@@ -810,11 +810,29 @@ def _scales_per_row(x, scale, block_size):
     return scale.dtype == torch.bfloat16 and tuple(scale.shape) == want and scale.is_contiguous()
 
 
-# Up to this many activation rows (one pass of ``vq_gemm_mx_rows``) the weight is streamed straight from its codes.
-# Measured on a B200, us, streamed / before: int8 codes in blocks of 16, 4096 x 4096: 18.6 / 69 for 7 rows, 25 / 70 for
-# 32, 51 / 74 for 64 in two passes; 14336 x 4096: 35 / 72 for 7, 70 / 73 for 32; 512 x 4096: 15 / 30 for 7.  16-entry
-# lookup codes in blocks of 64, 4096 x 4096: 23 / 39 for 7 rows, 31 / 40 for 32, 62 / 40 for 64.
+# Up to this many activation rows (one pass of ``vq_gemm_mx_rows``) the weight may be streamed straight from its codes.
 MX_STREAM_ROWS = 32
+
+
+def _stream_pays(rows, n, k, lookup):
+    """Whether the streamed weight beats the tensor-core GEMM (with the block scales in its main loop or behind a
+    read-back pass, whichever that takes).
+
+    Measured on a B200, us, streamed / GEMM, over N = 512 .. 128256 and K = 128 .. 14336.  Up to 24 rows it always does,
+    from 7.6 / 9.4 (512 x 128, 24 rows) and 17 / 68 (4096 x 4096, 7 rows) to 375 / 444 (128256 x 4096, 24 rows).  With
+    25 to 32 rows the streamed time grows by about 1.1 us per million weights beyond ten, and the GEMM's in steps:
+    * codes that are values: 45 / 70 (8448 x 4096), 72 / 74 (14336 x 4096); from N = 16384 on it wins where the GEMM's last
+      wave of 74 CTA pairs is not nearly full: 102 / 137 (22016 x 4096: 86 tiles), 125 / 136 (28672 x 4096: 112 tiles)
+      against 159 / 137 (16384 x 8192: 64 tiles), 90 / 75 (18944 x 4096: 74), 480 / 448 (128256 x 4096: 501);
+    * 16-entry lookups, whose GEMM decodes the weight first and then runs at 128 rows: 56 / 58 (9216 x 4096), 75 / 76
+      (10240 x 5120), 130 / 165 (12288 x 10752), 229 / 238 (14336 x 14336) against 82 / 77 (14336 x 4096), 122 / 103
+      (22016 x 4096), 173 / 156 (16384 x 8192)."""
+    if rows <= 24:
+        return True
+    if lookup:
+        return n <= 10240 or k > 8960
+    tiles = -(-n // 256)
+    return n < 16384 or tiles < 0.8 * 74 * -(-tiles // 74)
 
 
 def _level_table(code, entries):
@@ -840,7 +858,7 @@ def _mx_gemm_few_rows(native, a, b, bias, input_scale, weight_scale, block_size,
     if a.shape[-1] != k or k == 0 or n == 0 or k % 32 or k % block_size or k >= 1 << 30:
         return None
     rows = a.numel() // k
-    if rows == 0 or rows > MX_STREAM_ROWS:
+    if rows == 0 or rows > MX_STREAM_ROWS or not _stream_pays(rows, n, k, weight_code is not None):
         return None
     if not (_scales_per_row(a, input_scale, block_size) and _scales_per_row(b, weight_scale, block_size)
             and _level_table(input_code, 0) and _level_table(weight_code, 16)):
