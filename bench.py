@@ -933,7 +933,7 @@ class C3:
         cos, sin = W.rope_tables(self.cached, self.shape, dev)
         self.rope = (cos[-1].contiguous(), sin[-1].contiguous())
         self.x = [W.make_hidden_states(800 + 10 * rank + i, self.batch, self.shape, dev) for i in range(self.n_sets)]
-        self.launches_per_step = self.layers * W.Mxnf4DecodeLayer.LAUNCHES + 2
+        self.launches_per_step = self.layers * W.Mxnf4DecodeLayer.LAUNCHES + 3
         self.h2d_bytes = self.batch * self.shape.hidden * 2
         self.d2h_bytes = self.batch * self.shape.vocab * 2
         self._run(self.x[0])
@@ -1114,6 +1114,7 @@ class C5:
                 self.launches += 1
             self._mark("hessian")
             hinv = G.hessian_inverse_chol(h, self.calibration, 0.01)
+            self.launches += 3 * (k // 128)   # loading h, then diagonal block, panel and (but for the last) update a step
             del h
             self._mark("cholesky")
             out = G.sweep(w, hinv, 128, self.qmap, affine_range=(0.0, 15.0))

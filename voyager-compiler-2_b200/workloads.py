@@ -483,8 +483,9 @@ class Mxnf4DecodeLayer:
         self.residual_scale = residual_scale
         self.ln1, self.ln2 = weights["ln1"], weights["ln2"]
 
-    # kernels of this package per step: 4 quantize_mx, 4 linears, RoPE + append, the attention, 2 residual casts + adds
-    LAUNCHES = 12
+    # kernels of this package per step: 4 quantize_mx, 4 linears (each after the kernel that clears its counters), RoPE +
+    # append, the attention, 2 residual casts + adds
+    LAUNCHES = 16
 
     def _linear(self, x, name):
         from . import packed as P
