@@ -23,7 +23,7 @@
 // 64-position units, and the row maxima, the sums and the partial outputs are exchanged through distributed
 // shared memory, in rank order.  The newest positions belong to the last CTA; their count is padded to a multiple of 16
 // with scores of minus infinity, so any count from 16 on
-// runs here.  8 heads x 1013 positions (batch 1): 14.6 us with eight CTAs a head, where the window of 53 positions sent the
+// runs here.  8 heads x 1013 positions (batch 1): 14.6 us with four CTAs a head, where the window of 53 positions sent the
 // step through ten torch operators (55 us) before; 128 heads x 4096 positions take 53 us unsplit.
 //
 // Fragment layouts (lane = 4 g + t): A a0 = rows g, columns 2t, 2t+1; a2 = columns 2t+8, 2t+9 (a1, a3 are

@@ -23,7 +23,7 @@ namespace {
 // 64-element group, whose four scale bytes its first lane writes as one word.  Two blocks per thread are in flight.
 // The tensor-wide scale is `global_scale`, or follows from `amax` (and is then written to t_out).
 //
-// HBM-bound at 2 bytes in and 0.56 out per element: computing a block's scale once (two threads shared a block
+// Bound by instruction issue (ALU 76 %, DRAM 38 %; 2 bytes in and 0.56 out per element): computing a block's scale once (two threads shared a block
 // before) and testing the sixteen quotients' distance from a rounding boundary together took 8192 x 14336 from
 // 188 to 82 us (3.7 TB/s).
 constexpr int kCastBlocks = 2;

@@ -5,9 +5,10 @@
 //
 // Each takes two passes over the matrix: the tensor-wide amax (of the rotated transpose too, which is not stored), then
 // one kernel that reads 64 x 128 tiles and writes both packed forms.  HBM moves 2 x 2 bytes in and 2 x 0.56 out per
-// element; what bounds the rotated pass beside it is the rotation, 16 float32 FMAs per element in the operator's order,
-// issued as f32x2 over two output columns with the matrix broadcast from shared memory.  It is done once per pass: a
-// stored rotated transpose would cost 4 bytes per element more.
+// element and is 10 to 25 % busy: the amax pass waits for its loads, the casts are bound by instruction issue (ALU 61 %;
+// 30 instructions per element of a square weight, 78 of a rotated, stochastically rounded pair).  The rotation, 16
+// float32 FMAs per element in the operator's order, is issued as f32x2 over two output columns with the matrix
+// broadcast from shared memory, once per pass: a stored rotated transpose would cost 4 bytes per element more.
 //
 // 4096 x 4096: a rotated pair 62 us (96 with both forms stochastically rounded) and a square weight 33 us; as operators
 // of their own (rotate, transpose, amax, quantize, pack, the level table rebuilt and read by the host) the three casts
