@@ -272,7 +272,10 @@ __device__ __noinline__ uint4 quotients8_exact(uint4 x, float s) {
 // (quotients too small for its argument cast to a zero of their sign either way); 4 x 4 bytes are transposed in registers
 // and go to shared memory as words, exclusive-ored so that a warp's stores and 16-byte reads touch every bank once.
 // 4096 x 4096 with both outputs and the maximum (64 MB): 17.5 us, 25.7 as 64 x 64 tiles with a byte store per element.
-template <bool E4M3>
+// Bound by instruction issue (79 %; DRAM 34 %).  4095 x 4096, where the transposed rows begin at any byte: 28.4 us, 39 as
+// 64 x 64 tiles.
+// ANY: T is no multiple of 4.
+template <bool E4M3, bool ANY>
 __global__ void __launch_bounds__(512, 2)
 cast_transpose_kernel(const uint4* __restrict__ x, uint8_t* __restrict__ out, uint8_t* __restrict__ codes,
                       int* __restrict__ amax_bits, int T, int heads, int d, int64_t ldx, const void* __restrict__ scale,
@@ -332,27 +335,50 @@ cast_transpose_kernel(const uint4* __restrict__ x, uint8_t* __restrict__ out, ui
     if ((threadIdx.x & 31) == 0) atomicMax(&block_max, local);
   }
   __syncthreads();
-  const int piece = threadIdx.x & 7;   // 16 bytes of a column
+  const int n = min(128, T - t0);   // the tile's share of a transposed row
+  if (!ANY || n <= 32) {
+    const int piece = threadIdx.x & 7;   // 16 bytes of a column
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int j = (threadIdx.x >> 3) + 64 * u, s = (j >> 3) * 2;
-    if (j0 + j >= d) continue;
-    uint4 c = *reinterpret_cast<const uint4*>(&tile[j][4 * (piece ^ (s >> 2))]);
-    if (s & 2) c = make_uint4(c.z, c.w, c.x, c.y);
-    const int t = t0 + piece * 16;
-    uint8_t* dst = out + ((int64_t)h * d + j0 + j) * T + t;
-    if ((T & 15) == 0) {
-      if (t < T) *reinterpret_cast<uint4*>(dst) = c;
-    } else {
+    for (int u = 0; u < 2; ++u) {
+      const int j = (threadIdx.x >> 3) + 64 * u, s = (j >> 3) * 2;
+      if (j0 + j >= d) continue;
+      uint4 c = *reinterpret_cast<const uint4*>(&tile[j][4 * (piece ^ (s >> 2))]);
+      if (s & 2) c = make_uint4(c.z, c.w, c.x, c.y);
+      const int t = t0 + piece * 16;
+      uint8_t* dst = out + ((int64_t)h * d + j0 + j) * T + t;
       const uint32_t w[4] = {c.x, c.y, c.z, c.w};
-      if ((T & 3) == 0) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (t + 4 * q < T) reinterpret_cast<uint32_t*>(dst)[q] = w[q];
-      } else {
+      if (ANY) {
 #pragma unroll
         for (int q = 0; q < 16; ++q)
           if (t + q < T) dst[q] = (uint8_t)(w[q >> 2] >> (8 * (q & 3)));
+      } else if ((T & 15) == 0) {
+        if (t < T) *reinterpret_cast<uint4*>(dst) = c;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (t + 4 * q < T) reinterpret_cast<uint32_t*>(dst)[q] = w[q];
+      }
+    }
+  } else {
+    // rows that begin anywhere: a warp writes a column's run as whole aligned words, shifted together from two of the
+    // tile's, and the few bytes before the first and behind the last singly.  (4096 tokens are 13.8 us, 4095 20.8 so and 60
+    // with 16 byte stores per thread, which the shortest runs above still take: they wait less.)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t col[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) col[u] = tile[warp + 16 * u][lane ^ (((warp + 16 * u) >> 3) * 2)];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int j = warp + 16 * u;
+      if (j0 + j >= d) continue;
+      uint8_t* dst = out + ((int64_t)h * d + j0 + j) * T + t0;
+      const int head = min((int)(-reinterpret_cast<intptr_t>(dst) & 3), n), words = (n - head) >> 2, body = head + 4 * words;
+      const uint32_t next = __shfl_down_sync(0xFFFFFFFFu, col[u], 1);
+      if (lane < words) *reinterpret_cast<uint32_t*>(dst + head + 4 * lane) = __funnelshift_r(col[u], next, 8 * head);
+      if (n > 4 * words) {
+        const int at = lane < head ? lane : body + lane - head;   // the single bytes: [0, head) and [body, n)
+        const uint32_t w = __shfl_sync(0xFFFFFFFFu, col[u], (at >> 2) & 31);
+        if (at < n && (at < head || at >= body)) dst[at] = (uint8_t)(w >> (8 * (at & 3)));
       }
     }
   }
@@ -753,14 +779,19 @@ extern "C" int vq_transpose_quantize_fp8(const void* x, void* out, void* codes, 
   if (d % 8 == 0 && ldx % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
       (reinterpret_cast<uintptr_t>(codes) & 7) == 0) {
     const dim3 tiles((unsigned)((T + 127) / 128), (unsigned)((d + 127) / 128), (unsigned)heads);
-    if (format == VQ_IN_E4M3)
-      cast_transpose_kernel<true><<<tiles, 512, 0, st>>>(static_cast<const uint4*>(x), static_cast<uint8_t*>(out),
-                                                         static_cast<uint8_t*>(codes), static_cast<int*>(amax_bits), (int)T,
-                                                         (int)heads, (int)d, ldx, scale, scale_dtype);
-    else
-      cast_transpose_kernel<false><<<tiles, 512, 0, st>>>(static_cast<const uint4*>(x), static_cast<uint8_t*>(out),
-                                                          static_cast<uint8_t*>(codes), static_cast<int*>(amax_bits),
-                                                          (int)T, (int)heads, (int)d, ldx, scale, scale_dtype);
+    const bool any = (T & 3) != 0;
+#define VQ_CAST(F, ANY)                                                                                                   \
+  cast_transpose_kernel<F, ANY><<<tiles, 512, 0, st>>>(static_cast<const uint4*>(x), static_cast<uint8_t*>(out),          \
+                                                       static_cast<uint8_t*>(codes), static_cast<int*>(amax_bits), (int)T, \
+                                                       (int)heads, (int)d, ldx, scale, scale_dtype)
+    if (format == VQ_IN_E4M3) {
+      if (any) VQ_CAST(true, true);
+      else VQ_CAST(true, false);
+    } else {
+      if (any) VQ_CAST(false, true);
+      else VQ_CAST(false, false);
+    }
+#undef VQ_CAST
     return check_launch("cast_transpose_kernel");
   }
   dim3 grid((unsigned)((T + 63) / 64), (unsigned)((d + 63) / 64), (unsigned)heads);
