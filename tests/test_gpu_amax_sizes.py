@@ -1,4 +1,4 @@
-"""The tensor maximum over sizes on both sides of one load a thread."""
+"""The tensor maximum over sizes on both sides of one load a thread, and codebook read-backs around the table's threshold."""
 
 import pytest
 import torch
@@ -23,3 +23,15 @@ def test_amax_finds_the_largest_anywhere(n, where):
         N.check(N.lib().vq_amax(x.data_ptr(), 0, n, out.data_ptr(), torch.cuda.current_stream().cuda_stream))
         want = x[at].abs().float()
         assert torch.equal(out, want) or (bool(out.isnan()) and bool(want.isnan()))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 64), (15, 4096), (16, 4096), (31, 2112), (32, 2112)])
+def test_read_back_through_a_codebook(rows, cols):
+    import voyager_b200 as vb
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    codes = torch.randint(0, 16, (rows, cols), generator=g, device="cuda")
+    levels = torch.randn(16, generator=g, device="cuda").bfloat16()
+    scale = torch.randn(rows, cols // 64, generator=g, device="cuda").bfloat16()
+    got = torch.ops.quantized_ops.dequantize_mx(codes.bfloat16(), scale, 64, levels)
+    assert torch.equal(got, levels[codes] * scale.repeat_interleave(64, 1))
