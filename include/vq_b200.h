@@ -658,6 +658,13 @@ int vq_gemm_lut4(const void* a, int64_t lda, const void* a_scale, const void* a_
                  const void* w_packed, const void* w_scale, const void* w_levels, int block_size, void* out,
                  int out_dtype, int64_t N, int64_t K, const void* alpha, int alpha_dtype, const void* bias,
                  int bias_dtype, float* workspace, int* counters, void* stream);
+/* The same on counters that the caller has cleared (vq_clear_counters: n ints) since they were last used, so that the
+ * products of one step need one clearing. */
+int vq_gemm_lut4_cleared(const void* a, int64_t lda, const void* a_scale, const void* a_levels, int n_a_levels, int64_t M,
+                         const void* w_packed, const void* w_scale, const void* w_levels, int block_size, void* out,
+                         int out_dtype, int64_t N, int64_t K, const void* alpha, int alpha_dtype, const void* bias,
+                         int bias_dtype, float* workspace, int* counters, void* stream);
+int vq_clear_counters(int* counters, int64_t n, void* stream);
 
 /* linear_mx (ops/quantized.py:662-723) for at most 32 activation rows on the operator's own storage: a [M, K] and w
  * [N, K] bfloat16 codes with bfloat16 scales per `block_size` elements of K ([M, K / bs], [N, K / bs]); a_levels / w_levels:

@@ -151,3 +151,32 @@ def test_special_scales_and_scales_anywhere(m, n, k, bs, coded, off):
         again = vb.packed.linear_lut4(a, packed, input_scale=sa, input_code=levels, out_dtype=torch.float32)
         assert torch.equal(again.isnan(), want.isnan()) and torch.equal(again.isinf(), want.isinf())
         assert bool(((again.double() - want).abs() <= bound)[finite].all())
+
+
+@pytest.mark.parametrize("m", [1, 16, 32])
+def test_one_clearing_for_a_step(m):
+    """Products on counters cleared together are the products that clear their own, also when captured and replayed."""
+    import voyager_b200 as vb
+
+    P = vb.packed
+    weights = [_packed(vb, n, k, 64, n) for n, k in ((1000, 2048), (24, 4096), (4096, 1024))]
+    xs = [torch.randn(m, w.shape[1], generator=torch.Generator(device="cuda").manual_seed(i), device="cuda").bfloat16()
+          for i, w in enumerate(weights)]
+    want = [P.linear_lut4(x, w, out_dtype=torch.float32) for x, w in zip(xs, weights)]
+
+    def step():
+        return [P.linear_counted(x, w, c, out_dtype=torch.float32) for x, w, c in zip(xs, weights, P.step_counters(weights))]
+
+    assert all(torch.equal(a, b) for a, b in zip(step(), want))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step()
+    for _ in range(3):
+        for t in out:
+            t.fill_(float("nan"))
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(out, want))
+    counters = P.step_counters(weights)
+    for bad in (counters[1], counters[0].float(), counters[0].cpu()):
+        with pytest.raises(ValueError):
+            P.linear_counted(xs[0], weights[0], bad)

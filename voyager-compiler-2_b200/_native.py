@@ -128,6 +128,9 @@ SIGNATURES = {
     "vq_gemm_lut4_workspace_floats": [_I64, _I64, _I64],
     "vq_gemm_lut4_counters": [_I64],
     "vq_gemm_lut4": [_P, _I64, _P, _P, _I, _I64, _P, _P, _P, _I, _P, _I, _I64, _I64, _P, _I, _P, _I, _P, _P, _P],
+    "vq_gemm_lut4_cleared": [_P, _I64, _P, _P, _I, _I64, _P, _P, _P, _I, _P, _I, _I64, _I64, _P, _I, _P, _I, _P, _P,
+                             _P],
+    "vq_clear_counters": [_P, _I64, _P],
     "vq_pack_lut4": [_P, _P, _I64, _I64, _P, _P],
     "vq_kivi_decode_attention": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I64, _I64, _I64, _F, _P],
     "vq_kivi_write_2bit": [_P, _P, _P, _P, _I64, _I64, _I64, _I, _I64, ctypes.POINTER(VqRound), _P],

@@ -587,6 +587,14 @@ int lut4_status(int reset) {
 }
 }  // namespace vq
 
+extern "C" int vq_clear_counters(int* counters, int64_t n, void* stream) {
+  VQ_REQUIRE(n >= 0 && n < (1ll << 31), "vq_clear_counters: bad extent");
+  if (n == 0) return VQ_OK;
+  VQ_REQUIRE(counters, "vq_clear_counters: null argument");
+  clear_counters_kernel<<<(unsigned)((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(counters, (int)n);
+  return check_launch("clear_counters_kernel");
+}
+
 // How a product is cut: 8 * NT activation rows, weight tiles of 8 * RG rows, K slices, CTAs per slice.
 struct Lut4Plan {
   int nt, rg, tiles, steps, slices, ctas, max_parts, lda_s;
@@ -628,7 +636,7 @@ static bool lut4_launchable(const Lut4Plan& q) { return q.slices <= 65535 && (in
 
 // The cut, tensor maps and launch of a product whose operands stand in `p`.
 template <bool WIDE>
-static int launch_row_stream(Lut4Params p, cudaStream_t st) {
+static int launch_row_stream(Lut4Params p, bool clear, cudaStream_t st) {
   const int64_t M = p.M, N = p.N, K = p.K;
   const Lut4Plan q = lut4_plan(M, N, K, WIDE);
   p.tiles = q.tiles; p.steps = q.steps; p.slices = q.slices; p.ctas = q.ctas; p.max_parts = q.max_parts; p.lda_s = q.lda_s;
@@ -656,9 +664,9 @@ static int launch_row_stream(Lut4Params p, cudaStream_t st) {
     cudaFuncSetAttribute(gemm_lut4_kernel<WIDE, 3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
     cudaFuncSetAttribute(gemm_lut4_kernel<WIDE, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem);
   }
-  // cleared by every call and not by the last launch's tiles: a launch that gave up leaves some of them counted in part
-  clear_counters_kernel<<<(unsigned)((q.tiles + 255) / 256), 256, 0, st>>>(p.counters, q.tiles);
-  if (int e = check_launch("clear_counters_kernel")) return e;
+  // cleared for every launch and not by the last one's tiles: a launch that gave up leaves some of them counted in part
+  if (clear)
+    if (int e = vq_clear_counters(p.counters, q.tiles, st)) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)q.ctas, (unsigned)q.slices);
   cfg.blockDim = dim3(L4_THREADS);
@@ -668,7 +676,7 @@ static int launch_row_stream(Lut4Params p, cudaStream_t st) {
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = clear ? 1 : 0;
   const cudaError_t e = q.nt == 1   ? cudaLaunchKernelEx(&cfg, gemm_lut4_kernel<WIDE, 1, 4>, map_w, map_s, p)
                         : q.nt == 2 ? cudaLaunchKernelEx(&cfg, gemm_lut4_kernel<WIDE, 2, 4>, map_w, map_s, p)
                         : q.nt == 3 ? cudaLaunchKernelEx(&cfg, gemm_lut4_kernel<WIDE, 3, 2>, map_w, map_s, p)
@@ -733,7 +741,7 @@ int vq_gemm_mx_rows(const void* a, const void* a_scale, const void* a_levels, in
   // the tiles' counters belong to this call: products of several streams may run at the same time
   p.counters = static_cast<int*>(workspace);
   p.workspace = reinterpret_cast<float*>(p.counters + lut4_plan(M, N, K, true).tiles);
-  return launch_row_stream<true>(p, static_cast<cudaStream_t>(stream));
+  return launch_row_stream<true>(p, true, static_cast<cudaStream_t>(stream));
 }
 
 int vq_pack_lut4(const void* codes, void* packed, int64_t rows, int64_t K, int* bad, void* stream) {
@@ -746,7 +754,7 @@ int vq_pack_lut4(const void* codes, void* packed, int64_t rows, int64_t K, int* 
   return check_launch("pack_lut4_kernel");
 }
 
-int vq_gemm_lut4(const void* a, int64_t lda, const void* a_scale, const void* a_levels, int n_a_levels, int64_t M,
+static int gemm_lut4(bool clear, const void* a, int64_t lda, const void* a_scale, const void* a_levels, int n_a_levels, int64_t M,
                  const void* w_packed, const void* w_scale, const void* w_levels, int block_size, void* out,
                  int out_dtype, int64_t N, int64_t K, const void* alpha, int alpha_dtype, const void* bias,
                  int bias_dtype, float* workspace, int* counters, void* stream) {
@@ -771,7 +779,23 @@ int vq_gemm_lut4(const void* a, int64_t lda, const void* a_scale, const void* a_
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.bs = block_size; p.lda = lda;
   p.alpha = alpha; p.alpha_dt = alpha_dtype; p.bias = bias; p.bias_dt = bias_dtype;
   p.workspace = workspace; p.counters = counters;
-  return launch_row_stream<false>(p, static_cast<cudaStream_t>(stream));
+  return launch_row_stream<false>(p, clear, static_cast<cudaStream_t>(stream));
+}
+
+int vq_gemm_lut4(const void* a, int64_t lda, const void* a_scale, const void* a_levels, int n_a_levels, int64_t M,
+                 const void* w_packed, const void* w_scale, const void* w_levels, int block_size, void* out,
+                 int out_dtype, int64_t N, int64_t K, const void* alpha, int alpha_dtype, const void* bias,
+                 int bias_dtype, float* workspace, int* counters, void* stream) {
+  return gemm_lut4(true, a, lda, a_scale, a_levels, n_a_levels, M, w_packed, w_scale, w_levels, block_size, out, out_dtype, N, K,
+                   alpha, alpha_dtype, bias, bias_dtype, workspace, counters, stream);
+}
+
+int vq_gemm_lut4_cleared(const void* a, int64_t lda, const void* a_scale, const void* a_levels, int n_a_levels, int64_t M,
+                         const void* w_packed, const void* w_scale, const void* w_levels, int block_size, void* out,
+                         int out_dtype, int64_t N, int64_t K, const void* alpha, int alpha_dtype, const void* bias,
+                         int bias_dtype, float* workspace, int* counters, void* stream) {
+  return gemm_lut4(false, a, lda, a_scale, a_levels, n_a_levels, M, w_packed, w_scale, w_levels, block_size, out, out_dtype, N, K,
+                   alpha, alpha_dtype, bias, bias_dtype, workspace, counters, stream);
 }
 
 }  // extern "C"

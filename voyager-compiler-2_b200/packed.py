@@ -78,13 +78,35 @@ def _scratch(device, m, n, k):
     return torch.empty(floats + int(lib.vq_gemm_lut4_counters(n)), dtype=torch.float32, device=device), floats
 
 
+def step_counters(weights):
+    """Cleared tile counters for one product with each of ``weights`` (on one device), as one tensor per weight: a step of
+    several products clears once (2 us) where each ``linear_lut4`` clears its own (1.5 to 3 us)."""
+    sizes = [int(N.lib().vq_gemm_lut4_counters(w.shape[0])) for w in weights]
+    counters = torch.empty(sum(sizes), dtype=torch.int32, device=weights[0].codes.device)
+    _clear(counters)
+    return counters.split(sizes)
+
+
 @N.device_guarded
+def _clear(counters):
+    N.check(N.lib().vq_clear_counters(counters.data_ptr(), counters.numel(), _stream()), "vq_clear_counters")
+
+
 def linear_lut4(input: torch.Tensor, weight: PackedLUT4Weight, bias: Optional[torch.Tensor] = None, *,
                 input_scale: Optional[torch.Tensor] = None, input_code: Optional[torch.Tensor] = None,
                 alpha: Optional[torch.Tensor] = None, out_dtype=None) -> torch.Tensor:
     """``linear_mx(input, W, bias, input_scale=, weight_scale=, block_size=, input_code=, weight_code=, alpha=)``
     for a packed ``W``.  ``input [..., K]`` is bfloat16: values, or codebook indices when ``input_code`` is given;
     ``input_scale [..., K / block_size]``."""
+    return linear_counted(input, weight, None, bias, input_scale=input_scale, input_code=input_code, alpha=alpha,
+                          out_dtype=out_dtype)
+
+
+@N.device_guarded
+def linear_counted(input: torch.Tensor, weight: PackedLUT4Weight, counters: Optional[torch.Tensor],
+                   bias: Optional[torch.Tensor] = None, *, input_scale: Optional[torch.Tensor] = None,
+                   input_code: Optional[torch.Tensor] = None, alpha: Optional[torch.Tensor] = None, out_dtype=None):
+    """``linear_lut4`` on counters from ``step_counters`` (one product each), or on its own."""
     n, k = weight.shape
     if input.dtype != torch.bfloat16 or input.shape[-1] != k:
         raise NotImplementedError(f"linear_lut4 takes bfloat16 activations of width {k}")
@@ -113,11 +135,17 @@ def linear_lut4(input: torch.Tensor, weight: PackedLUT4Weight, bias: Optional[to
     if bias is not None:
         bias = bias.contiguous()
     out = torch.empty((m, n), dtype=dtype, device=x.device)
+    lib = N.lib()
     work, floats = _scratch(x.device, m, n, k)
-    N.check(N.lib().vq_gemm_lut4(x.data_ptr(), k, _ptr(scale), _ptr(code), 0 if code is None else code.numel(), m,
-                                 weight.codes.data_ptr(), weight.scale.data_ptr(), weight.levels.data_ptr(),
-                                 weight.block_size, out.data_ptr(), _dtype_id(dtype), n, k, _ptr(alpha),
-                                 0 if alpha is None else _dtype_id(alpha.dtype), _ptr(bias),
-                                 0 if bias is None else _dtype_id(bias.dtype), work.data_ptr(),
-                                 work.data_ptr() + 4 * floats, _stream()), "vq_gemm_lut4")
+    if counters is None:
+        call, count_ptr = lib.vq_gemm_lut4, work.data_ptr() + 4 * floats
+    else:
+        if counters.dtype != torch.int32 or counters.numel() < lib.vq_gemm_lut4_counters(n) or not counters.is_contiguous() \
+                or counters.device != x.device:
+            raise ValueError("counters are one tensor of step_counters' result")
+        call, count_ptr = lib.vq_gemm_lut4_cleared, counters.data_ptr()
+    N.check(call(x.data_ptr(), k, _ptr(scale), _ptr(code), 0 if code is None else code.numel(), m, weight.codes.data_ptr(),
+                 weight.scale.data_ptr(), weight.levels.data_ptr(), weight.block_size, out.data_ptr(), _dtype_id(dtype), n, k,
+                 _ptr(alpha), 0 if alpha is None else _dtype_id(alpha.dtype), _ptr(bias),
+                 0 if bias is None else _dtype_id(bias.dtype), work.data_ptr(), count_ptr, _stream()), "vq_gemm_lut4")
     return out.reshape(*lead, n)

@@ -483,16 +483,16 @@ class Mxnf4DecodeLayer:
         self.residual_scale = residual_scale
         self.ln1, self.ln2 = weights["ln1"], weights["ln2"]
 
-    # kernels of this package per step: 4 quantize_mx, 4 linears (each after the kernel that clears its counters), RoPE +
-    # append, the attention, 2 residual casts + adds
-    LAUNCHES = 16
+    # kernels of this package per step: 4 quantize_mx, 4 linears and the clearing of their counters, RoPE + append, the
+    # attention, 2 residual casts + adds
+    LAUNCHES = 13
 
-    def _linear(self, x, name):
+    def _linear(self, x, name, counters):
         from . import packed as P
 
         t = self.t
         s, c = torch.ops.quantized_ops.quantize_mx(x, t["index"], [-1], 64, 31.0, False, t["e5m3"], t["mid"])
-        return P.linear_lut4(c, self.w[name], input_scale=s, input_code=t["levels"])
+        return P.linear_counted(c, self.w[name], counters[name], input_scale=s, input_code=t["levels"])
 
     def _through_fp8(self, x):
         q = torch.ops.quantized_ops.quantize(x, self.residual_scale, None, None, None, self.t["e4m3"])
@@ -516,7 +516,11 @@ class Mxnf4DecodeLayer:
         def rotate(v):
             return v * cos + torch.cat([-v[..., half:], v[..., :half]], -1) * sin
 
-        qkv = self._linear(F.rms_norm(x, (sh.hidden,), self.ln1, sh.eps), "qkv")
+        from . import packed as P
+
+        names = ("qkv", "o", "gate_up", "down")
+        counters = dict(zip(names, P.step_counters([self.w[n] for n in names])))   # this step's own
+        qkv = self._linear(F.rms_norm(x, (sh.hidden,), self.ln1, sh.eps), "qkv", counters)
         k_res, v_res = self.cache["k_res"], self.cache["v_res"]
         if self.fused_attention:
             from . import kivi as KV
@@ -540,10 +544,10 @@ class Mxnf4DecodeLayer:
             p = torch.softmax(scores * (1.0 / math.sqrt(d)), -1, dtype=torch.float32).to(x.dtype)
             tm = k_main.shape[-2]
             ctx = torch.matmul(p[..., :tm], v_main) + torch.matmul(p[..., tm:], v_res)
-        x1 = self._residual_add(x, self._linear(ctx.reshape(B, hq * d), "o"))
-        gu = self._linear(F.rms_norm(x1, (sh.hidden,), self.ln2, sh.eps), "gate_up")
+        x1 = self._residual_add(x, self._linear(ctx.reshape(B, hq * d), "o", counters))
+        gu = self._linear(F.rms_norm(x1, (sh.hidden,), self.ln2, sh.eps), "gate_up", counters)
         inter = gu.shape[-1] // 2
-        return self._residual_add(x1, self._linear(F.silu(gu[:, :inter]) * gu[:, inter:], "down"))
+        return self._residual_add(x1, self._linear(F.silu(gu[:, :inter]) * gu[:, inter:], "down", counters))
 
     __call__ = forward
 
